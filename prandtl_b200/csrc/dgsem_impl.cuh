@@ -22,6 +22,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "dgsem_kernels.cuh"
 
@@ -145,19 +146,12 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *dst, double v
     atomicMax(dst, (unsigned long long)__double_as_longlong(v));
 }
 
-// Block-wide max of per-thread values, one atomic per CTA.
-template <int THREADS>
-__device__ __forceinline__ void block_max_to(unsigned long long *dst, double v, double *sred) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) sred[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = sred[0];
-        for (int q = 1; q < (THREADS + 31) / 32; ++q) m = fmax(m, sred[q]);
-        atomic_max_pos(dst, m);
-    }
+// The same, skipping the atomic when *dst already holds at least v: *dst only
+// grows, so a stale read can cost an atomic but never lose a maximum.
+__device__ __forceinline__ void atomic_max_seen(unsigned long long *dst, double v) {
+    const unsigned long long seen = *reinterpret_cast<volatile unsigned long long *>(dst);
+    if (v >= 0.0 && (unsigned long long)__double_as_longlong(v) <= seen) return;
+    atomic_max_pos(dst, v);
 }
 
 // Hoisted per-node primitive table in shared memory: H[k*ND + node].
@@ -1693,7 +1687,7 @@ struct FieldRows {
     }
 };
 
-template <int DIM, int NP, typename W, bool VC, bool CURV = false>
+template <int DIM, int NP, typename W, bool VC, bool LINES, bool CURV = false>
 __device__ __forceinline__ void lift_element(const ElemIO &a, const PhysParams &P, int e, bool active,
                                              const W *sT, W *sElem, int n) {
     using S = Shape<DIM, NP>;
@@ -1886,10 +1880,16 @@ __device__ __forceinline__ void lift_element(const ElemIO &a, const PhysParams &
 #pragma unroll
             for (int r = 0; r < DIM; ++r) Vc[r][f] += adj[r][cc] * val;
         });
+        // LINES: per element [DIM][NF-1][position along the line][line], so that the
+        // lanes that own the lines of direction r read row r in order
 #pragma unroll
-        for (int r = 0; r < DIM; ++r)
+        for (int r = 0; r < DIM; ++r) {
+            const long long at = (long long)e * (DIM * (NF - 1) * ND) + r * (NF - 1) * ND + c[r] * (ND / NP) +
+                                 line_index<DIM, NP>(r, c);
 #pragma unroll
-            for (int f = 1; f < NF; ++f) gout[(r * (NF - 1) + f - 1) * Ndof + gnode] = Vc[r][f];
+            for (int f = 1; f < NF; ++f)
+                gout[LINES ? at + (f - 1) * ND : (r * (NF - 1) + f - 1) * Ndof + gnode] = Vc[r][f];
+        }
     } else {
 #pragma unroll
         for (int q = 0; q < DIM; ++q)
@@ -1963,7 +1963,7 @@ lift_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_
     io.fnn = m.fnn;
     io.snor = nullptr;
     using LL = LiftLayout<DIM, NP, Out, CURV>;
-    lift_element<DIM, NP, Out, VC, CURV>(io, P, active ? e_raw : m.E - 1, active, smem,
+    lift_element<DIM, NP, Out, VC, VC && !CURV && sizeof(Out) == 8, CURV>(io, P, active ? e_raw : m.E - 1, active, smem,
                                          smem + LL::TABW + el * LL::PER_ELEM, n);
 }
 
@@ -2001,7 +2001,7 @@ lift_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_const
         __syncthreads();
         const int e_raw = e0 + el;
         const bool active = e_raw < E;
-        lift_element<DIM, NP, Out, VC>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT,
+        lift_element<DIM, NP, Out, VC, VC && sizeof(Out) == 8>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT,
                                    sE + el * LiftLayout<DIM, NP, Out>::PER_ELEM, nn);
     }
 }
@@ -2054,6 +2054,14 @@ inline bool smem_attribute_lost(cudaError_t err, size_t bytes, std::atomic<unsig
     return true;
 }
 
+}   // namespace
+}   // namespace prandtl
+
+#include "dgsem_line.cuh"
+
+namespace prandtl {
+namespace {
+
 template <int DIM, int NP, bool NS, bool VC, typename Real, bool CURV>
 cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
                           cudaStream_t s) {
@@ -2070,6 +2078,10 @@ cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &
     }
     return cudaErrorInvalidValue;
 }
+// The FP64 forms on affine meshes run by lines (dgsem_line.cuh), but for
+// Navier-Stokes with gradients and the axisymmetric form.
+template <bool NS, bool VC, typename Real>
+constexpr bool line_form() { return sizeof(Real) == 8 && (VC || !NS); }
 // non-affine meshes (m.ngeo set) run the per-node-geometry kernels (FP64, or FP32-bulk Euler)
 template <int DIM, int NP, bool NS, bool VC, typename Real>
 cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
@@ -2078,7 +2090,12 @@ cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams 
         if constexpr (sizeof(Real) == 8 || !NS) return rhs_launch_np<DIM, NP, NS, VC, Real, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
     }
-    return rhs_launch_np<DIM, NP, NS, VC, Real, false>(m, a, P, T, s);
+    if constexpr (line_form<NS, VC, Real>()) {   // by lines, but for the axisymmetric form
+        if (DIM == 3 || NS || !m.rad) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
+    }
+    if constexpr (sizeof(Real) == 4 || (NS && !VC) || (DIM == 2 && !NS))
+        return rhs_launch_np<DIM, NP, NS, VC, Real, false>(m, a, P, T, s);
+    else return cudaErrorNotSupported;
 }
 template <int DIM, int NP, typename Out, bool VC, bool CURV>
 cudaError_t lift_launch_np(const MeshDev &m, const LiftArgs &a, const PhysParams &P, const OpTables &T,
@@ -2108,8 +2125,11 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
 
 // Batch kernels: `prepare` sets the shared-memory attribute (outside any stream
 // capture) and reports the resident CTAs per SM; `launch` only launches.
-template <int DIM, int NP, bool NS, bool VC, typename Real, int V>
+template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_prepare_np(BatchKernelInfo *info) {
+    if constexpr (line_form<NS, VC, Real>()) {
+        return LineBatch<DIM, NP, NS, FEAT, V>::prepare(info);
+    } else {
     using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
     const size_t sm = rhs_batch_smem<DIM, NP, NS, VC, Real, V>();
     cudaError_t err = cudaFuncSetAttribute(rhs_batch_kernel<DIM, NP, NS, VC, Real, V>,
@@ -2126,13 +2146,18 @@ cudaError_t rhs_batch_prepare_np(BatchKernelInfo *info) {
     info->regs = fa.numRegs;
     info->elems_per_item = LY::ITEM_ELEMS;
     return cudaSuccess;
+    }
 }
-template <int DIM, int NP, bool NS, bool VC, typename Real, int V>
+template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
                                 cudaStream_t s) {
-    using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
-    rhs_batch_kernel<DIM, NP, NS, VC, Real, V><<<grid, LY::THREADS, rhs_batch_smem<DIM, NP, NS, VC, Real, V>(), s>>>(c, st, T);
-    return cudaGetLastError();
+    if constexpr (line_form<NS, VC, Real>()) {
+        return LineBatch<DIM, NP, NS, FEAT, V>::launch(grid, c, st, T, s);
+    } else {
+        using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
+        rhs_batch_kernel<DIM, NP, NS, VC, Real, V><<<grid, LY::THREADS, rhs_batch_smem<DIM, NP, NS, VC, Real, V>(), s>>>(c, st, T);
+        return cudaGetLastError();
+    }
 }
 template <int DIM, int NP, typename Out, bool VC>
 cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
@@ -2191,16 +2216,18 @@ cudaError_t lift_dispatch(int order, const MeshDev &m, const LiftArgs &a, const 
     PRANDTL_ORDER_SWITCH((lift_launch_any<DIM, NP, Out, VC>(m, a, P, T, s)))
 }
 template <int DIM, typename Real, bool NS, bool VC>
-cudaError_t rhs_batch_prepare(int order, int variant, BatchKernelInfo *info) {
+cudaError_t rhs_batch_prepare(int order, int variant, bool feat, BatchKernelInfo *info) {
     PRANDTL_ORDER_SWITCH(([&]() -> cudaError_t {
-        PRANDTL_VARIANT_SWITCH(return (rhs_batch_prepare_np<DIM, NP, NS, VC, Real, VV>(info)))
+        PRANDTL_VARIANT_SWITCH(return feat ? (rhs_batch_prepare_np<DIM, NP, NS, VC, Real, VV, true>(info))
+                                           : (rhs_batch_prepare_np<DIM, NP, NS, VC, Real, VV, false>(info)))
     }()))
 }
 template <int DIM, typename Real, bool NS, bool VC>
-cudaError_t rhs_batch_launch(int order, int variant, int grid, const BatchClassDev &c, const BatchStage &st,
-                             const OpTables &T, cudaStream_t s) {
+cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const BatchClassDev &c,
+                             const BatchStage &st, const OpTables &T, cudaStream_t s) {
     PRANDTL_ORDER_SWITCH(([&]() -> cudaError_t {
-        PRANDTL_VARIANT_SWITCH(return (rhs_batch_launch_np<DIM, NP, NS, VC, Real, VV>(grid, c, st, T, s)))
+        PRANDTL_VARIANT_SWITCH(return feat ? (rhs_batch_launch_np<DIM, NP, NS, VC, Real, VV, true>(grid, c, st, T, s))
+                                           : (rhs_batch_launch_np<DIM, NP, NS, VC, Real, VV, false>(grid, c, st, T, s)))
     }()))
 }
 template <int DIM, typename Out, bool VC>
@@ -2217,8 +2244,8 @@ cudaError_t lift_batch_launch(int order, int grid, const BatchClassDev &c, const
 #define PRANDTL_INSTANTIATE_RHS(DIMV, REAL, NSV, VCV)                                                   \
     template cudaError_t rhs_dispatch<DIMV, REAL, NSV, VCV>(int, const MeshDev &, const RhsArgs &,      \
                                                             const PhysParams &, const OpTables &, cudaStream_t); \
-    template cudaError_t rhs_batch_prepare<DIMV, REAL, NSV, VCV>(int, int, BatchKernelInfo *);          \
-    template cudaError_t rhs_batch_launch<DIMV, REAL, NSV, VCV>(int, int, int, const BatchClassDev &,   \
+    template cudaError_t rhs_batch_prepare<DIMV, REAL, NSV, VCV>(int, int, bool, BatchKernelInfo *);          \
+    template cudaError_t rhs_batch_launch<DIMV, REAL, NSV, VCV>(int, int, bool, int, const BatchClassDev &,   \
                                                                 const BatchStage &, const OpTables &, cudaStream_t);
 #define PRANDTL_INSTANTIATE_LIFT(DIMV, OUT, VCV)                                                        \
     template cudaError_t lift_dispatch<DIMV, OUT, VCV>(int, const MeshDev &, const LiftArgs &,          \

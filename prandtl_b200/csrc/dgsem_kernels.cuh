@@ -121,11 +121,13 @@ bool order_supported(int dim, int order);
 // Batch kernels of one class.  `variant` in [0, batch_num_variants()) picks the
 // RHS launch shape.  `vc` selects the Navier-Stokes form that passes
 // contravariant viscous fluxes from the lifting to the RHS (quirks = 1) instead
-// of primitive gradients (quirks = 0).  prepare_* must run outside stream capture.
+// of primitive gradients (quirks = 0).  `feat`: the class's solves have blending
+// or boundary conditions (their code is compiled out of the other kernels).  prepare_* must run outside stream capture.
 int batch_num_variants();
-cudaError_t batch_prepare_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, BatchKernelInfo *info);
+cudaError_t batch_prepare_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat,
+                              BatchKernelInfo *info);
 cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, BatchKernelInfo *info);
-cudaError_t batch_launch_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, int grid,
+cudaError_t batch_launch_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat, int grid,
                              const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s);
 cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, int grid, const BatchClassDev &c,
                               const BatchStage &st, const OpTables &T, cudaStream_t s);
@@ -164,10 +166,10 @@ template <int DIM, typename Out, bool VC>
 cudaError_t lift_dispatch(int order, const MeshDev &m, const LiftArgs &a, const PhysParams &P,
                           const OpTables &T, cudaStream_t s);
 template <int DIM, typename Real, bool NS, bool VC>
-cudaError_t rhs_batch_prepare(int order, int variant, BatchKernelInfo *info);
+cudaError_t rhs_batch_prepare(int order, int variant, bool feat, BatchKernelInfo *info);
 template <int DIM, typename Real, bool NS, bool VC>
-cudaError_t rhs_batch_launch(int order, int variant, int grid, const BatchClassDev &c, const BatchStage &st,
-                             const OpTables &T, cudaStream_t s);
+cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const BatchClassDev &c,
+                             const BatchStage &st, const OpTables &T, cudaStream_t s);
 template <int DIM, typename Out, bool VC>
 cudaError_t lift_batch_prepare(int order, BatchKernelInfo *info);
 template <int DIM, typename Out, bool VC>

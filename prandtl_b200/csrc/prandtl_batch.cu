@@ -117,7 +117,11 @@ Layout solve_layout(int dim, int order, int E, int F, bool ns, bool blending, bo
     return L;
 }
 
-int class_key(int dim, int order, bool ns, bool vc) { return ((dim * 16 + order) * 2 + (ns ? 1 : 0)) * 2 + (vc ? 1 : 0); }
+// feat: blending or boundary conditions, whose kernels differ; a class of its
+// own, so that a solve runs the same kernel whatever else the batch holds
+int class_key(int dim, int order, bool ns, bool vc, bool feat) {
+    return (((dim * 16 + order) * 2 + (ns ? 1 : 0)) * 2 + (vc ? 1 : 0)) * 2 + (feat ? 1 : 0);
+}
 
 struct Solve {
     bool used = false;
@@ -134,6 +138,7 @@ constexpr int MAX_VARIANTS = 8;
 struct Class {
     int dim = 0, order = 0;
     bool ns = false, vc = false;   // vc: NS with contravariant viscous fluxes (quirks = 1)
+    bool feat = false;             // blending or boundary conditions
     OpTables T{};
     std::vector<int> ids;        // slot -> solve id
     int *d_buf = nullptr;        // ids[cap] | prefix[cap + 1] | hdr[4]
@@ -352,8 +357,8 @@ prandtl_status up_copy(prandtl_batch *b, void *dst, const void *src, size_t n) {
     return PRANDTL_OK;
 }
 
-prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc, Class **out) {
-    const int key = class_key(dim, order, ns, vc);
+prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc, bool feat, Class **out) {
+    const int key = class_key(dim, order, ns, vc, feat);
     auto it = b->classes.find(key);
     if (it != b->classes.end()) { *out = &it->second; return PRANDTL_OK; }
     Class c;
@@ -361,12 +366,13 @@ prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc,
     c.order = order;
     c.ns = ns;
     c.vc = vc;
+    c.feat = feat;
     build_tables(order, c.T);
     const bool fp32 = b->cfg.precision == 1;
     int first_ok = -1;
     for (int v = 0; v < b->nvar; ++v) {
         c.ms[v] = -1.0;
-        BCK(b, batch_prepare_rhs(dim, order, ns, vc, fp32, v, &c.rinfo[v]), "prepare batch rhs kernel");
+        BCK(b, batch_prepare_rhs(dim, order, ns, vc, fp32, v, feat, &c.rinfo[v]), "prepare batch rhs kernel");
         if (c.rinfo[v].blocks_per_sm > 0 && first_ok < 0) first_ok = v;
     }
     if (first_ok < 0) return bfail(b, PRANDTL_EUNSUPPORTED, "no RHS launch shape fits this device");
@@ -402,7 +408,7 @@ prandtl_status enqueue_step(prandtl_batch *b, cudaStream_t s) {
                 BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, grid, c.dev, st, c.T, s), "batch lift launch");
             }
             const int grid = c.rinfo[c.variant].blocks_per_sm * b->num_sms;
-            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, c.variant, grid, c.dev, st, c.T, s),
+            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, c.variant, c.feat, grid, c.dev, st, c.T, s),
                 "batch rhs launch");
         }
     }
@@ -442,7 +448,7 @@ prandtl_status tune_step(prandtl_batch *b, int v) {
             const int cv = c.rinfo[v].blocks_per_sm > 0 ? v : c.variant;
             const int grid = c.rinfo[cv].blocks_per_sm * b->num_sms;
             BCK(b, cudaEventRecord(b->tev[q + 2], b->stream), "event");
-            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, cv, grid, c.dev, st, c.T, b->stream),
+            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, cv, c.feat, grid, c.dev, st, c.T, b->stream),
                 "batch rhs launch");
             BCK(b, cudaEventRecord(b->tev[q + 3], b->stream), "event");
             q += 4;
@@ -741,11 +747,11 @@ prandtl_status admit_prepared(prandtl_batch *b, const prandtl_mesh_desc *md, con
     BCK(b, cudaSetDevice(b->device), "cudaSetDevice");
     const int dim = md->dim, order = md->order, E = md->num_elements, F = md->num_faces;
     const bool ns = cfg->parabolic != 0, fp32 = b->cfg.precision == 1, blend = cfg->blending != 0;
-    const bool vc = ns && cfg->quirks != 0;
+    const bool vc = ns && cfg->quirks != 0, feat = blend || cfg->num_bcs > 0;
     const Layout L = solve_layout(dim, order, E, F, ns, blend, fp32, cfg->num_bcs);
     if (b->free_ids.empty()) return bfail(b, PRANDTL_ENOMEM, "solve table full");
     Class *c = nullptr;
-    if ((st = get_class(b, dim, order, ns, vc, &c)) != PRANDTL_OK) return st;
+    if ((st = get_class(b, dim, order, ns, vc, feat, &c)) != PRANDTL_OK) return st;
     size_t off = 0;
     if (!b->alloc.alloc(L.total, &off))
         return bfail(b, PRANDTL_ENOMEM, "arena has no room: need " + std::to_string(L.total) +
@@ -757,7 +763,7 @@ prandtl_status admit_prepared(prandtl_batch *b, const prandtl_mesh_desc *md, con
     s.dim = dim;
     s.order = order;
     s.ns = ns;
-    s.key = class_key(dim, order, ns, vc);
+    s.key = class_key(dim, order, ns, vc, feat);
     s.E = E;
     s.nf = dim + 2;
     s.gamma = cfg->gamma;
@@ -1164,10 +1170,10 @@ prandtl_status prandtl_batch_tune(prandtl_batch *b, int reps) {
             c.ms[v] = -1.0;
             if (c.rinfo[v].blocks_per_sm <= 0) continue;
             const int grid = c.rinfo[v].blocks_per_sm * b->num_sms;
-            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, v, grid, c.dev, st0, c.T, b->stream), "tune rhs");
+            BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, v, c.feat, grid, c.dev, st0, c.T, b->stream), "tune rhs");
             BCK(b, cudaEventRecord(b->ev0, b->stream), "event");
             for (int r = 0; r < reps; ++r)
-                BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, v, grid, c.dev, st0, c.T, b->stream), "tune rhs");
+                BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, v, c.feat, grid, c.dev, st0, c.T, b->stream), "tune rhs");
             BCK(b, cudaEventRecord(b->ev1, b->stream), "event");
             if ((st = bwait(b)) != PRANDTL_OK) return st;
             float ms = 0.f;
@@ -1186,8 +1192,9 @@ prandtl_status prandtl_batch_class_info(prandtl_batch *b, int dim, int order, in
                                         int *n_variants, double *ms, double *lift_ms) {
     if (!b) return PRANDTL_EINVAL;
     std::lock_guard<std::mutex> lk(b->mu);
-    auto it = b->classes.find(class_key(dim, order, parabolic != 0, parabolic != 0));
-    if (it == b->classes.end()) it = b->classes.find(class_key(dim, order, parabolic != 0, false));
+    auto it = b->classes.end();
+    for (int q = 0; q < 4 && it == b->classes.end(); ++q)   // plain solves first, vc before gradients
+        it = b->classes.find(class_key(dim, order, parabolic != 0, parabolic != 0 && !(q & 1), (q & 2) != 0));
     if (it == b->classes.end()) return bfail(b, PRANDTL_EINVAL, "no such class in this batch");
     if (variant) *variant = it->second.variant;
     if (n_variants) *n_variants = b->nvar;

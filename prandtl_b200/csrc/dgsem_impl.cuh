@@ -1687,7 +1687,7 @@ struct FieldRows {
     }
 };
 
-template <int DIM, int NP, typename W, bool VC, bool LINES, bool CURV = false>
+template <int DIM, int NP, typename W, bool VC, bool CURV = false>
 __device__ __forceinline__ void lift_element(const ElemIO &a, const PhysParams &P, int e, bool active,
                                              const W *sT, W *sElem, int n) {
     using S = Shape<DIM, NP>;
@@ -1880,16 +1880,10 @@ __device__ __forceinline__ void lift_element(const ElemIO &a, const PhysParams &
 #pragma unroll
             for (int r = 0; r < DIM; ++r) Vc[r][f] += adj[r][cc] * val;
         });
-        // LINES: per element [DIM][NF-1][position along the line][line], so that the
-        // lanes that own the lines of direction r read row r in order
 #pragma unroll
-        for (int r = 0; r < DIM; ++r) {
-            const long long at = (long long)e * (DIM * (NF - 1) * ND) + r * (NF - 1) * ND + c[r] * (ND / NP) +
-                                 line_index<DIM, NP>(r, c);
+        for (int r = 0; r < DIM; ++r)
 #pragma unroll
-            for (int f = 1; f < NF; ++f)
-                gout[LINES ? at + (f - 1) * ND : (r * (NF - 1) + f - 1) * Ndof + gnode] = Vc[r][f];
-        }
+            for (int f = 1; f < NF; ++f) gout[(r * (NF - 1) + f - 1) * Ndof + gnode] = Vc[r][f];
     } else {
 #pragma unroll
         for (int q = 0; q < DIM; ++q)
@@ -1963,7 +1957,7 @@ lift_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_
     io.fnn = m.fnn;
     io.snor = nullptr;
     using LL = LiftLayout<DIM, NP, Out, CURV>;
-    lift_element<DIM, NP, Out, VC, VC && !CURV && sizeof(Out) == 8, CURV>(io, P, active ? e_raw : m.E - 1, active, smem,
+    lift_element<DIM, NP, Out, VC, CURV>(io, P, active ? e_raw : m.E - 1, active, smem,
                                          smem + LL::TABW + el * LL::PER_ELEM, n);
 }
 
@@ -2001,7 +1995,7 @@ lift_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_const
         __syncthreads();
         const int e_raw = e0 + el;
         const bool active = e_raw < E;
-        lift_element<DIM, NP, Out, VC, VC && sizeof(Out) == 8>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT,
+        lift_element<DIM, NP, Out, VC>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT,
                                    sE + el * LiftLayout<DIM, NP, Out>::PER_ELEM, nn);
     }
 }
@@ -2120,7 +2114,9 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
         if constexpr (sizeof(Out) == 8) return lift_launch_np<DIM, NP, Out, VC, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
     }
-    return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
+    if constexpr (line_form<true, VC, Out>())
+        return m.bcs ? lift_line_launch<DIM, NP, true>(m, a, P, T, s) : lift_line_launch<DIM, NP, false>(m, a, P, T, s);
+    else return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
 }
 
 // Batch kernels: `prepare` sets the shared-memory attribute (outside any stream
@@ -2128,7 +2124,8 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
 template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_prepare_np(BatchKernelInfo *info) {
     if constexpr (line_form<NS, VC, Real>()) {
-        return LineBatch<DIM, NP, NS, FEAT, V>::prepare(info);
+        using L = LineShape<DIM, NP>;
+        return line_batch_prepare<L>((const void *)rhs_line_batch_kernel<DIM, NP, NS, FEAT, V>, line_batch_smem<L>(), info);
     } else {
     using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
     const size_t sm = rhs_batch_smem<DIM, NP, NS, VC, Real, V>();
@@ -2152,7 +2149,9 @@ template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
                                 cudaStream_t s) {
     if constexpr (line_form<NS, VC, Real>()) {
-        return LineBatch<DIM, NP, NS, FEAT, V>::launch(grid, c, st, T, s);
+        using L = LineShape<DIM, NP>;
+        rhs_line_batch_kernel<DIM, NP, NS, FEAT, V><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, T);
+        return cudaGetLastError();
     } else {
         using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
         rhs_batch_kernel<DIM, NP, NS, VC, Real, V><<<grid, LY::THREADS, rhs_batch_smem<DIM, NP, NS, VC, Real, V>(), s>>>(c, st, T);
@@ -2161,6 +2160,10 @@ cudaError_t rhs_batch_launch_np(int grid, const BatchClassDev &c, const BatchSta
 }
 template <int DIM, int NP, typename Out, bool VC>
 cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
+    if constexpr (line_form<true, VC, Out>()) {
+        using L = LiftLineShape<DIM, NP>;
+        return line_batch_prepare<L>((const void *)lift_line_batch_kernel<DIM, NP>, line_batch_smem<L>(), info);
+    } else {
     using S = LiftBatchShape<DIM, NP, Out>;
     const size_t sm = lift_batch_smem<DIM, NP, Out>();
     cudaError_t err = cudaFuncSetAttribute(lift_batch_kernel<DIM, NP, Out, VC>,
@@ -2177,12 +2180,18 @@ cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
     info->regs = fa.numRegs;
     info->elems_per_item = S::EPB;
     return cudaSuccess;
+    }
 }
 template <int DIM, int NP, typename Out, bool VC>
 cudaError_t lift_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
                                  cudaStream_t s) {
-    using S = LiftBatchShape<DIM, NP, Out>;
-    lift_batch_kernel<DIM, NP, Out, VC><<<grid, S::THREADS, lift_batch_smem<DIM, NP, Out>(), s>>>(c, st, T);
+    if constexpr (line_form<true, VC, Out>()) {
+        using L = LiftLineShape<DIM, NP>;
+        lift_line_batch_kernel<DIM, NP><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, T);
+    } else {
+        using S = LiftBatchShape<DIM, NP, Out>;
+        lift_batch_kernel<DIM, NP, Out, VC><<<grid, S::THREADS, lift_batch_smem<DIM, NP, Out>(), s>>>(c, st, T);
+    }
     return cudaGetLastError();
 }
 

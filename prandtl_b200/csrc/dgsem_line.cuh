@@ -64,11 +64,14 @@ struct LineShape {
 // line's sums and primitives take 80 (3D, Np = 4); at 128 registers the 3D
 // kernels spill in the two-point fluxes (32^3 Np = 4 Navier-Stokes 157 -> 228 us,
 // 24^3 Euler 52 -> 60 us), and more than 168 gives up resident warps (2D Np = 5
-// Euler 22.9 -> 25.4 us at 255).
-// The batch's other two launch shapes (V = 1, 2) have 255 and 128.
-template <int DIM, int NP, int V = 0>
+// Euler 22.9 -> 25.4 us, 3D Np = 5 Euler 69 -> 81 us at 255).  The 3D Np = 5
+// Navier-Stokes kernel alone, whose viscous rows come on top, is faster with 255
+// (20^3: 123 -> 97 us).  The batch's other two launch shapes (V = 1, 2) have 255
+// and 128.
+template <int DIM, int NP, bool NS, int V = 0>
 constexpr int line_min_blocks() {
-    return cmax(1, 65536 / ((V == 0 ? 168 : V == 1 ? 255 : 128) * LineShape<DIM, NP>::THREADS));
+    return cmax(1, 65536 / ((V == 1 || (V == 0 && NS && DIM == 3 && NP == 5) ? 255 : V == 2 ? 128 : 168) *
+                            LineShape<DIM, NP>::THREADS));
 }
 
 // Logarithmic mean of x, y > 0 in the form q = (x+y) / (2 mean), with
@@ -674,36 +677,330 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
 }
 
 
-// One-shot kernel.  blockDim may be any multiple of 32 up to THREADS when
+// ------------------------------------------------------------ BR1 lifting
+// The lifting of the Navier-Stokes form with contravariant viscous fluxes, by
+// lines as above: a lane differentiates its line's entropy variables and adds
+// the line's two face jumps; the nodes' lanes (the lines of the last direction)
+// form the primitive gradients and the viscous rows.  The entropy variables are
+// relative to the element's node 0 (constants drop out of derivatives and
+// jumps), so that the logarithms are of ratios near one, by series.  The
+// node-by-node form (lift_element) spent 30 % of its FP64 instructions on
+// logarithms, left half of the threads idle on every second face item and read
+// every node's variables 3 Np times; it was bound by latency and barriers at
+// 19 warps per SM.  Measured: 32^3 Np = 4 179 -> 109 us (HBM floor 43 us for
+// 285 MB), 20^3 Np = 5 90 -> 65 us, 2D 120x60 Np = 5 unchanged at 17 us.
+template <int DIM, int NP>
+struct LiftLineShape : LineShape<DIM, NP> {
+    using L = LineShape<DIM, NP>;
+    // rows: entropy variables [NF], derivatives along the first DIM-1 directions [DIM-1][NF];
+    // then the neighbour table and the geometry
+    static constexpr int NBR = DIM * L::NF * L::ROW, GEO = NBR + 2 * DIM, END = GEO + DIM * DIM + 1;
+    static constexpr int PER_ELEM = END + (L::STRIDE16 + 16 - END % 16) % 16;
+};
+
+// ln(x / x0) for x, x0 > 0.
+__device__ __forceinline__ double log_ratio(double x, double x0) {
+    const double f = (x - x0) * rcp(x + x0), u = f * f;
+    double q = 1.0 / 11.0;
+#pragma unroll
+    for (int k = 9; k >= 1; k -= 2) q = fma(q, u, 1.0 / k);   // truncation u^6/13 < 1e-19
+    if (!(u < 1e-3)) q = log_q_far(x0, x, f, u);
+    return 2.0 * f * q;
+}
+// Entropy variables (BasicOperations.cpp:81-104) of state s relative to those of
+// the reference node (rho, p, beta = rho/p, beta |v|^2 / 2).
+struct LineRef {
+    double rho, p, beta, bvsq;
+};
+template <int DIM>
+__device__ __forceinline__ LineRef line_ref(const double *s, const PhysParams &P) {
+    const double r = rcp(s[0]);
+    double mm = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) mm = fma(s[1 + d], s[1 + d], mm);
+    LineRef R;
+    R.rho = s[0];
+    R.p = P.gammaM1 * fma(-0.5 * mm, r, s[1 + DIM]);
+    R.beta = s[0] * rcp(R.p);
+    R.bvsq = R.beta * (0.5 * mm * r * r);
+    return R;
+}
+template <int DIM>
+__device__ __forceinline__ void line_entropy(const double *s, const PhysParams &P, const LineRef &R, double *v) {
+    const double r = rcp(s[0]);
+    double vel[DIM], vv = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        vel[d] = s[1 + d] * r;
+        vv = fma(vel[d], vel[d], vv);
+    }
+    const double p = P.gammaM1 * fma(-0.5 * s[0], vv, s[1 + DIM]);
+    const double beta = s[0] * rcp(p);
+    const double ds = fma(-P.gamma, log_ratio(s[0], R.rho), log_ratio(p, R.p));
+    v[0] = -fma(ds, P.gammaM1Inverse, fma(0.5 * beta, vv, -R.bvsq));
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) v[1 + d] = beta * vel[d];
+    v[1 + DIM] = R.beta - beta;
+}
+// The lifting's boundary value minus the inner trace's, as boundary_lift_trace
+// defines it (fixed mode): 1/2 (v(outer) - v1), at the no-slip walls v_wall - v1.
+template <int DIM>
+__device__ __noinline__ void line_lift_boundary(const BcDev &bc, const PhysParams &P, const double *s1,
+                                                const double *nor, double *lf) {
+    constexpr int NF = DIM + 2;
+    double v1[NF];
+    conserv2entropy<DIM, double>(s1, P, v1);
+    if (bc.type == BC_NOSLIP_ADIABATIC || bc.type == BC_NOSLIP_ISOTHERMAL) {
+        const bool adiab = bc.type == BC_NOSLIP_ADIABATIC;
+        const double b = adiab ? -v1[NF - 1] : bc.vT;
+        lf[0] = 0.0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) lf[1 + d] = bc.wall_vel[d] * b - v1[1 + d];
+        lf[NF - 1] = adiab ? 0.0 : -bc.vT - v1[NF - 1];
+        return;
+    }
+    double c[NF], s2[NF], v2[NF], nn = 0.0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) c[f] = s1[f];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) nn += nor[d] * nor[d];
+    bc_outer_state<DIM>(bc, c, nor, sqrt(nn), P, s2);
+    conserv2entropy<DIM, double>(s2, P, v2);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) lf[f] = 0.5 * (v2[f] - v1[f]);
+}
+
+template <int DIM, int NP, bool BC, typename Sync>
+__device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysParams &P, const OpTables &T, int e, bool ok,
+                                                  double *sV, int ln, const Sync &sync) {
+    using L = LiftLineShape<DIM, NP>;
+    constexpr int ND = L::ND, NL = L::NL, NF = L::NF, ROW = L::ROW;
+    double *sG = sV + NF * ROW, *sGeo = sV + L::GEO;
+    int2 *sNbr = reinterpret_cast<int2 *>(sV + L::NBR);   // {element, local face}
+    const long long Ndof = a.Ndof, e0 = (long long)e * ND;
+    const int own0 = ln % NP + L::SY * (DIM == 2 ? 0 : ln / NP);
+    constexpr int own_st = DIM == 2 ? L::SY : L::SZ;
+    LineRef R{};
+    if (ok) {
+        constexpr int NG = (DIM * DIM + NL) / NL, NB = (2 * DIM + NL - 1) / NL;
+        int4 nb[NB];
+        double g[NG], s[NP][NF], s0[NF];
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            nb[k] = __ldg(a.nbr + (long long)e * (2 * DIM) + min(ln + k * NL, 2 * DIM - 1));
+#pragma unroll
+        for (int f = 0; f < NF; ++f) s0[f] = __ldg(a.u + f * Ndof + e0);
+#pragma unroll
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+            for (int f = 0; f < NF; ++f) s[i][f] = __ldg(a.u + f * Ndof + e0 + ln + NL * i);
+#pragma unroll
+        for (int k = 0; k < NG; ++k) g[k] = __ldg(a.geo + (long long)e * (DIM * DIM + 1) + min(ln + k * NL, DIM * DIM));
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            if (ln + k * NL < 2 * DIM)   // .y: local face, or ~(boundary condition) beside the face id
+                sNbr[ln + k * NL] = nb[k].x >= 0 ? make_int2(nb[k].x, nb[k].y) : make_int2(nb[k].z, ~nb[k].y);
+#pragma unroll
+        for (int k = 0; k < NG; ++k)
+            if (ln + k * NL < DIM * DIM + 1) sGeo[ln + k * NL] = g[k];
+        R = line_ref<DIM>(s0, P);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            double v[NF];
+            line_entropy<DIM>(s[i], P, R, v);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) sV[f * ROW + own0 + i * own_st] = v[f];
+        }
+    }
+    sync();
+
+    const double hw0 = 0.5 / T.w[0];
+    double gl[NP][NF];
+#pragma unroll 1
+    for (int dir = 0; dir < DIM; ++dir) {
+        if (ok) {
+            int sa, sb, st, ga, gb, gt;
+            line_strides<DIM>(dir, L::SY, L::SZ, sa, sb, st);
+            line_strides<DIM>(dir, NP, NP * NP, ga, gb, gt);
+            const int n0 = sa * (ln % NP) + sb * (ln / NP);
+            // neighbour traces of the line's faces (boundary faces: the own trace)
+            double s[2][NF];
+            int2 nb[2];
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                nb[side] = sNbr[2 * dir + side];
+                long long g = e0 + ga * (ln % NP) + gb * (ln / NP) + side * (NP - 1) * gt;
+                if (!BC || nb[side].y >= 0) {
+                    int na, nbs, nt;
+                    line_strides<DIM>(nb[side].y >> 1, NP, NP * NP, na, nbs, nt);
+                    g = (long long)nb[side].x * ND + na * (ln % NP) + nbs * (ln / NP) + (nb[side].y & 1) * (NP - 1) * nt;
+                }
+#pragma unroll
+                for (int f = 0; f < NF; ++f) s[side][f] = ldg_now(a.u + f * Ndof + g);
+            }
+            // derivative along the line: sum_l D(i, l) v_l
+            double v0[NF], v1[NF];
+#pragma unroll
+            for (int l = 0; l < NP; ++l) {
+                double v[NF];
+#pragma unroll
+                for (int f = 0; f < NF; ++f) v[f] = sV[f * ROW + n0 + l * st];
+#pragma unroll
+                for (int i = 0; i < NP; ++i)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) gl[i][f] = l == 0 ? T.D[i * NP] * v[f] : fma(T.D[i * NP + l], v[f], gl[i][f]);
+                if (l == 0)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) v0[f] = v[f];
+                if (l == NP - 1)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) v1[f] = v[f];
+            }
+            // + 1/(w0 J) 1/2 (v_neighbour - v_own) n at the ends (LiftingBR1.cpp:10-115); the outward
+            // scaled normal of an affine element's local face lf is (lf odd ? +1 : -1) times row lf/2 of
+            // adj(J), so the jump adds to the derivative along that row's direction
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                double vn[NF], jump[NF];
+                if (BC && nb[side].y < 0) {
+                    double in[NF], nor[DIM], lf[NF];
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) in[f] = s[side][f];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) nor[d] = __ldg(a.fnor + (long long)nb[side].x * DIM + d);
+                    line_lift_boundary<DIM>(a.bcs[~nb[side].y], P, in, nor, lf);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) jump[f] = 2.0 * lf[f];
+                } else {
+                    line_entropy<DIM>(s[side], P, R, vn);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) jump[f] = vn[f] - (side ? v1[f] : v0[f]);
+                }
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    if (side) gl[NP - 1][f] = fma(hw0, jump[f], gl[NP - 1][f]);
+                    else gl[0][f] = fma(-hw0, jump[f], gl[0][f]);
+                }
+            }
+            if (dir < DIM - 1) {
+                double *out = sG + dir * NF * ROW + n0;
+#pragma unroll
+                for (int i = 0; i < NP; ++i)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) out[f * ROW + i * st] = gl[i][f];
+            }
+        }
+    }
+    sync();
+    if (!ok) return;
+
+    // ---- node by node: gradients (grad1 adj / J, LiftingBR1.cpp:205-206), the chain rule
+    // and the contravariant viscous flux adj Fv^T, rows f = 1..NF-1, in line order
+    const double mJ = rcp(sGeo[DIM * DIM]);
+    double *gout = reinterpret_cast<double *>(a.grad) + (long long)e * (DIM * (NF - 1) * ND);
+    double adj[DIM][DIM];
+#pragma unroll
+    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+        for (int q = 0; q < DIM; ++q) adj[r][q] = sGeo[r * DIM + q];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int n = own0 + i * own_st;
+        double s[NF], g1[DIM][NF], g[DIM][NF], vel[DIM], Vc[DIM][NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) s[f] = __ldg(a.u + f * Ndof + e0 + ln + NL * i);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+#pragma unroll
+            for (int r = 0; r < DIM - 1; ++r) g1[r][f] = sG[(r * NF + f) * ROW + n];
+            g1[DIM - 1][f] = gl[i][f];
+        }
+#pragma unroll
+        for (int q = 0; q < DIM; ++q) {
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                double x = g1[0][f] * adj[0][q];
+#pragma unroll
+                for (int r = 1; r < DIM; ++r) x = fma(g1[r][f], adj[r][q], x);
+                g[q][f] = x * mJ;
+            }
+            entropygrad2primgrad<DIM, double>(s, P, g[q]);
+        }
+        const double rr = rcp(s[0]);
+        double vv = 0.0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            vel[d] = s[1 + d] * rr;
+            vv += vel[d] * vel[d];
+        }
+        const double p = P.gammaM1 * (s[NF - 1] - s[0] * (0.5 * vv));
+#pragma unroll
+        for (int r = 0; r < DIM; ++r)
+#pragma unroll
+            for (int f = 0; f < NF; ++f) Vc[r][f] = 0.0;
+        viscous_flux<DIM, double>(s[0], rr, vel, p, g, P, [&](int f, int cc, double val) {
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) Vc[r][f] = fma(adj[r][cc], val, Vc[r][f]);
+        });
+        const int c[3] = {ln % NP, DIM == 2 ? i : ln / NP, i};
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            double *out = gout + r * (NF - 1) * ND + c[r] * NL + line_index<DIM, NP>(r, c);
+#pragma unroll
+            for (int f = 1; f < NF; ++f) out[(f - 1) * ND] = Vc[r][f];
+        }
+    }
+}
+
+// A thread's element (slot el of the CTA, mesh element e) and line.
+template <typename L>
+struct LineLane {
+    int el, ln, e;
+    bool lane_ok;
+    __device__ __forceinline__ LineLane() {
+        const int x = L::WARP ? threadIdx.x & 31 : threadIdx.x;
+        el = x / L::NL;
+        ln = x - el * L::NL;
+        lane_ok = el < (L::WARP ? L::EPW : L::EPB);
+        if (!lane_ok) el = 0;
+        if (L::WARP) el += (threadIdx.x >> 5) * L::EPW;
+        e = blockIdx.x * (L::WARP ? (blockDim.x >> 5) * L::EPW : L::EPB) + el;
+    }
+};
+template <typename L>
+struct LineSync {
+    __device__ __forceinline__ void operator()() const {
+        if constexpr (L::WARP) __syncwarp();
+        else __syncthreads();
+    }
+};
+
+// One-shot kernels.  blockDim may be any multiple of 32 up to THREADS when
 // elements are packed into warps, THREADS otherwise.
 template <int DIM, int NP, bool NS, bool BLEND, bool BC>
-__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP>()))
+__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, NS>()))
 rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
     using L = LineShape<DIM, NP>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    int el, ln, epb;
-    bool lane_ok;
-    if constexpr (L::WARP) {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        el = lane / L::NL;
-        ln = lane - el * L::NL;
-        lane_ok = el < L::EPW;
-        el += w * L::EPW;
-        epb = (blockDim.x >> 5) * L::EPW;
-    } else {
-        el = threadIdx.x / L::NL;
-        ln = threadIdx.x - el * L::NL;
-        lane_ok = el < L::EPB;
-        epb = L::EPB;
-    }
-    const int e = blockIdx.x * epb + el;
-    const bool ok = lane_ok && e < m.E;
-    double *sH = reinterpret_cast<double *>(smem_raw) + (lane_ok ? el : 0) * L::PER_ELEM;
+    const LineLane<L> q;
+    const bool ok = q.lane_ok && q.e < m.E;
+    double *sH = reinterpret_cast<double *>(smem_raw) + q.el * L::PER_ELEM;
     const ElemIO io = io_from_args(m, a);
-    rhs_line_element<DIM, NP, NS, BLEND, BC>(io, P, T, ok ? e : 0, ok, sH, ln, [] {
-        if constexpr (L::WARP) __syncwarp();
-        else __syncthreads();
-    });
+    rhs_line_element<DIM, NP, NS, BLEND, BC>(io, P, T, ok ? q.e : 0, ok, sH, q.ln, LineSync<L>{});
+}
+template <int DIM, int NP, bool BC>
+__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, false>()))
+lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
+    using L = LiftLineShape<DIM, NP>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const LineLane<L> q;
+    const bool ok = q.lane_ok && q.e < m.E;
+    double *sV = reinterpret_cast<double *>(smem_raw) + q.el * L::PER_ELEM;
+    RhsArgs r{};
+    r.u = a.u;
+    r.grad = a.grad;
+    const ElemIO io = io_from_args(m, r);
+    lift_line_element<DIM, NP, BC>(io, P, T, ok ? q.e : 0, ok, sV, q.ln, LineSync<L>{});
 }
 
 // Persistent batch kernel: a fixed grid walks the class's work items, each the
@@ -711,10 +1008,8 @@ rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __gr
 // solve's element range is padded to BATCH_CHUNK in the class prefix; every
 // chunk holds ceil(BATCH_CHUNK / EPI) items, the last one shorter.  FEAT: the
 // class's solves have blending or boundary conditions.
-template <int DIM, int NP, bool NS, bool FEAT, int V>
-__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, V>()))
-rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
-    using L = LineShape<DIM, NP>;
+template <typename L, typename Element>
+__device__ __forceinline__ void line_batch_items(const BatchClassDev &c, const BatchStage &st, const Element &element) {
     constexpr int EPI = L::WARP ? L::EPW : L::EPB;                 // elements per item
     constexpr int IPC = (BATCH_CHUNK + EPI - 1) / EPI;             // items per chunk
     constexpr int SLOTS = L::WARP ? L::THREADS / 32 : 1;           // items in flight per CTA
@@ -725,10 +1020,7 @@ rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_c
     const int el = il / L::NL, ln = il - el * L::NL;
     const bool lane_ok = el < EPI;
     double *sH = reinterpret_cast<double *>(smem_raw + CTX_RESERVE) + (slot * EPI + (lane_ok ? el : 0)) * L::PER_ELEM;
-    auto sync = [] {
-        if constexpr (L::WARP) __syncwarp();
-        else __syncthreads();
-    };
+    const LineSync<L> sync{};
     const int n = c.hdr[0];
     const int total = n > 0 ? c.prefix[n] / BATCH_CHUNK * IPC : 0;
     for (int item = blockIdx.x * SLOTS + slot; item < total; item += gridDim.x * SLOTS) {
@@ -748,53 +1040,73 @@ rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_c
         }
         sync();
         const bool ok = lane_ok && e0 + el < E && in + el < BATCH_CHUNK;
-        rhs_line_element<DIM, NP, NS, FEAT, FEAT>(ctx->io, ctx->P, T, ok ? e0 + el : e0, ok, sH, ln, sync);
+        element(ctx->io, ctx->P, ok ? e0 + el : e0, ok, sH, ln, sync);
     }
 }
 template <int DIM, int NP, bool NS, bool FEAT, int V>
-struct LineBatch {
+__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, NS, V>()))
+rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
     using L = LineShape<DIM, NP>;
-    static constexpr size_t SMEM = CTX_RESERVE + sizeof(double) * (size_t)L::EPB * L::PER_ELEM;
-    static cudaError_t prepare(BatchKernelInfo *info) {
-        auto k = rhs_line_batch_kernel<DIM, NP, NS, FEAT, V>;
-        cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-        if (err != cudaSuccess) return err;
-        int nb = 0;
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, L::THREADS, SMEM);
-        if (err != cudaSuccess) return err;
-        cudaFuncAttributes fa{};
-        cudaFuncGetAttributes(&fa, k);
-        info->blocks_per_sm = nb;
-        info->threads = L::THREADS;
-        info->smem = (int)SMEM;
-        info->regs = fa.numRegs;
-        info->elems_per_item = L::WARP ? L::EPW : L::EPB;
-        return cudaSuccess;
-    }
-    static cudaError_t launch(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s) {
-        rhs_line_batch_kernel<DIM, NP, NS, FEAT, V><<<grid, L::THREADS, SMEM, s>>>(c, st, T);
-        return cudaGetLastError();
-    }
-};
-
-template <int DIM, int NP, bool NS, bool BLEND, bool BC>
-cudaError_t rhs_line_launch(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
-    using L = LineShape<DIM, NP>;
+    line_batch_items<L>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sH, int ln,
+                                   const LineSync<L> &sync) {
+        rhs_line_element<DIM, NP, NS, FEAT, FEAT>(io, P, T, e, ok, sH, ln, sync);
+    });
+}
+// (the lifting's boundary code is compiled into every batch kernel: one class
+// launch serves solves with and without boundary conditions)
+template <int DIM, int NP>
+__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, false>()))
+lift_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
+    using L = LiftLineShape<DIM, NP>;
+    line_batch_items<L>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sV, int ln,
+                                   const LineSync<L> &sync) {
+        lift_line_element<DIM, NP, true>(io, P, T, e, ok, sV, ln, sync);
+    });
+}
+template <typename L>
+cudaError_t line_batch_prepare(const void *k, size_t smem, BatchKernelInfo *info) {
+    cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    int nb = 0;
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, L::THREADS, smem);
+    if (err != cudaSuccess) return err;
+    cudaFuncAttributes fa{};
+    cudaFuncGetAttributes(&fa, k);
+    info->blocks_per_sm = nb;
+    info->threads = L::THREADS;
+    info->smem = (int)smem;
+    info->regs = fa.numRegs;
+    info->elems_per_item = L::WARP ? L::EPW : L::EPB;
+    return cudaSuccess;
+}
+template <typename L>
+constexpr size_t line_batch_smem() { return CTX_RESERVE + sizeof(double) * (size_t)L::EPB * L::PER_ELEM; }
+template <typename L, typename Kernel, typename Args>
+cudaError_t line_launch(Kernel k, std::atomic<unsigned> &smem_set, const MeshDev &m, const Args &a, const PhysParams &P,
+                        const OpTables &T, cudaStream_t s) {
     int threads = L::THREADS;
     if constexpr (L::WARP)   // small meshes: one-warp CTAs, so that every SM gets work
         while (threads > 32 && m.E < 148 * (threads / 32) * L::EPW) threads /= 2;
     const int epb = L::WARP ? threads / 32 * L::EPW : L::EPB;
     const size_t sm = sizeof(double) * (size_t)epb * L::PER_ELEM;
-    static std::atomic<unsigned> smem_set{0u};
     for (int attempt = 0; attempt < 2; ++attempt) {
-        cudaError_t err = smem_attribute_once((const void *)rhs_line_kernel<DIM, NP, NS, BLEND, BC>,
-                                              (int)sizeof(double) * L::EPB * L::PER_ELEM, smem_set);
+        cudaError_t err = smem_attribute_once((const void *)k, (int)sizeof(double) * L::EPB * L::PER_ELEM, smem_set);
         if (err != cudaSuccess) return err;
-        rhs_line_kernel<DIM, NP, NS, BLEND, BC><<<(m.E + epb - 1) / epb, threads, sm, s>>>(m, a, P, T);
+        k<<<(m.E + epb - 1) / epb, threads, sm, s>>>(m, a, P, T);
         err = cudaGetLastError();
         if (!smem_attribute_lost(err, sm, smem_set)) return err;
     }
     return cudaErrorInvalidValue;
+}
+template <int DIM, int NP, bool NS, bool BLEND, bool BC>
+cudaError_t rhs_line_launch(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
+    static std::atomic<unsigned> smem_set{0u};
+    return line_launch<LineShape<DIM, NP>>(rhs_line_kernel<DIM, NP, NS, BLEND, BC>, smem_set, m, a, P, T, s);
+}
+template <int DIM, int NP, bool BC>
+cudaError_t lift_line_launch(const MeshDev &m, const LiftArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
+    static std::atomic<unsigned> smem_set{0u};
+    return line_launch<LiftLineShape<DIM, NP>>(lift_line_kernel<DIM, NP, BC>, smem_set, m, a, P, T, s);
 }
 template <int DIM, int NP, bool NS>
 cudaError_t rhs_line_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {

@@ -661,7 +661,9 @@ __device__ __forceinline__ void boundary_flux(const BcDev &bc, const double *s_i
 // flux differencing, surface fluxes, gradients): double for the plain FP64
 // path, float for the FP32-bulk form.  Per-node primitives are always formed
 // in FP64 from the FP64 state, and the RK stage update is FP64.
-template <int DIM, int NP, bool NS, bool VC, typename Real, typename LY, bool CURV = false>
+// FEAT: the mesh may have boundary faces and the solve blending; their code is
+// compiled out of the other kernels, which miss the instruction cache less.
+template <int DIM, int NP, bool NS, bool VC, typename Real, typename LY, bool FEAT, bool CURV = false>
 __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P, int e, bool active,
                                             const Real *sT, const uint32_t *sPair, Real *sH, int li, int lane,
                                             int gid) {
@@ -758,7 +760,8 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 
     // ---- blending coefficient (PerssonPeraireIndicator.cpp:21-58, DGSEMOperator.cpp:60-80)
     Real alpha = 0;
-    if (P.blending) {
+    const bool blending = FEAT && P.blending;
+    if (blending) {
         Real *b0 = sF, *b1 = sF + ND;
 #pragma unroll 1
         for (int k = 0; k < NPL; ++k) {
@@ -849,8 +852,17 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 #pragma unroll
         for (int f = 0; f < NF; ++f) { dUi[k][f] = 0; dUv[k][f] = 0; }
 
+    // VC: row f (1..NF-1) of direction r at node n of element el.  Affine elements:
+    // in line order (lift_line_element), per element [DIM][NF-1][position along
+    // the line][line]; non-affine: [DIM][NF-1][Ndof]
+    auto visc_at = [&](long long el, int r, int f, int n) -> long long {
+        if (CURV) return (r * (NF - 1) + f - 1) * Ndof + el * ND + n;
+        int c[3];
+        node_coords<NP>(n, c);
+        return ((el * DIM + r) * (NF - 1) + f - 1) * ND + c[r] * S::NLINE + line_index<DIM, NP>(r, c);
+    };
     // ---- NS: contravariant viscous flux of every own node (flux_mat = adj * Fv^T, :632)
-    if constexpr (NS && VC) {
+    if constexpr (NS && VC && !LY::LINE) {   // (line tasks read their rows themselves)
         // formed by the lifting: rows f = 1..NF-1 of adj * Fv^T (the mass row is zero);
         // each lane's loads are all issued before the stores
         Real vrow[NPL][DIM][NF - 1];
@@ -861,7 +873,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
             for (int r = 0; r < DIM; ++r)
 #pragma unroll
                 for (int f = 1; f < NF; ++f)
-                    vrow[k][r][f - 1] = n < ND ? __ldg(grad + (r * (NF - 1) + f - 1) * Ndof + (long long)e * ND + n) : Real(0);
+                    vrow[k][r][f - 1] = n < ND ? __ldg(grad + visc_at(e, r, f, n)) : Real(0);
         }
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
@@ -873,7 +885,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
                     for (int f = 1; f < NF; ++f) sV[(r * LY::VROWS + f - LY::VOFF) * ND + n] = vrow[k][r][f - 1];
             }
         }
-    } else if constexpr (NS) {
+    } else if constexpr (NS && !VC) {
 #pragma unroll 1
         for (int k = 0; k < NPL; ++k) {
             const int n = li + k * GS;
@@ -920,7 +932,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
         //      reads them).  Q2 (quirks == 0, 3D): a zeta-line node's partners
         //      below it contribute the eta flux G(l) of DGSEMIntegrator.cpp:702.
         group_sync<GS>(gid);
-        const Real blend = P.blending ? Real(1) - alpha : Real(1);
+        const Real blend = blending ? Real(1) - alpha : Real(1);
         for (int t = li; t < DIM * S::NLINE; t += GS) {
             const int dir = t / S::NLINE, ln = t - dir * S::NLINE;
             int base, stride;
@@ -986,7 +998,9 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 #pragma unroll
             for (int l = 0; l < NP; ++l)
 #pragma unroll
-                for (int f = 1; f < NF; ++f) vv[l][f - 1] = sV[(dir * NF + f) * ND + base + l * stride];
+                for (int f = 1; f < NF; ++f)
+                    vv[l][f - 1] = VC ? __ldg(grad + (((long long)e * DIM + dir) * (NF - 1) + f - 1) * ND + l * S::NLINE + ln)
+                                      : sV[(dir * NF + f) * ND + base + l * stride];
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
                 Real *out = sV + dir * NF * ND + base + i * stride;
@@ -1120,7 +1134,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
                 Real v = -dUi[k][f];
-                if (P.blending) v *= (Real(1) - alpha);
+                if (blending) v *= (Real(1) - alpha);
                 if (NS) v += dUv[k][f];
                 acc[k][f] = v * mJn;
             }
@@ -1139,7 +1153,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
     }
 
     // ---- subcell first-order FV (DGSEMIntegrator.cpp:972-1196), skipped when alpha == 0
-    if (P.blending && alpha != Real(0)) {
+    if (blending && alpha != Real(0)) {
         Real fv[NPL][NF];
 #pragma unroll
         for (int dir = 0; dir < DIM; ++dir) {
@@ -1209,9 +1223,11 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
     };
     auto face_load = [&](int it, FaceIn &x) {
         const int lf = it / NFN, fa = it - lf * NFN;
-        const long long go = (long long)e * ND + face_node<DIM, NP>(lf, fa);
+        const int no = face_node<DIM, NP>(lf, fa);
         x.t = NBR_SMEM ? sNbr[lf] : __ldg(a.nbr + (long long)e * (2 * DIM) + lf);
-        const long long gs = x.t.x < 0 ? go : (long long)x.t.x * ND + face_node<DIM, NP>(x.t.y, fa);
+        const long long en = x.t.x < 0 ? e : x.t.x;
+        const int nn = x.t.x < 0 ? no : face_node<DIM, NP>(x.t.y, fa);
+        const long long gs = en * ND + nn;
 #pragma unroll
         for (int f = 0; f < NF; ++f) x.s[f] = __ldg(a.u + f * Ndof + gs);
 #pragma unroll
@@ -1222,8 +1238,8 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
             const int dd = lf >> 1, dn = x.t.x < 0 ? dd : x.t.y >> 1;
 #pragma unroll
             for (int f = 1; f < NF; ++f) {
-                x.vo[f - 1] = __ldg(grad + (dd * (NF - 1) + f - 1) * Ndof + go);
-                x.vn[f - 1] = __ldg(grad + (dn * (NF - 1) + f - 1) * Ndof + gs);
+                x.vo[f - 1] = __ldg(grad + visc_at(e, dd, f, no));
+                x.vn[f - 1] = __ldg(grad + visc_at(en, dn, f, nn));
             }
         }
     };
@@ -1244,7 +1260,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
         const long long go = (long long)e * ND + no;
         // 1 / (w0 J): non-affine elements take J at the face point (Elem1/Elem2 Weight())
         const Real awn = CURV ? Real(1.0 / (double(sW[0]) * ngeo(no, DIM * DIM))) : aw;
-        if (t.x < 0) {   // boundary face: the element is Elem1 (BdrFaceIntegrator.cpp:61-186)
+        if (FEAT && t.x < 0) {   // boundary face: the element is Elem1 (BdrFaceIntegrator.cpp:61-186)
             double sb[NF], nb[DIM];
             Real fb[NF], fv[NF];
 #pragma unroll
@@ -1502,7 +1518,7 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 
 // One-shot kernel: grid = ceil(E / EPB), one element per lane group.  CURV:
 // non-affine elements (per-node geometry; FP64, or FP32-bulk Euler).
-template <int DIM, int NP, bool NS, bool VC, typename Real, bool CURV>
+template <int DIM, int NP, bool NS, bool VC, typename Real, bool FEAT, bool CURV>
 __global__ void __launch_bounds__(RhsLayout<DIM, NP, NS, Real, 0, VC>::THREADS, (RhsLayout<DIM, NP, NS, Real, 0, VC>::MIN_BLOCKS))
 rhs_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
     using LY = RhsLayout<DIM, NP, NS, Real, 0, VC>;
@@ -1519,7 +1535,7 @@ rhs_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_co
     const int e_raw = blockIdx.x * LY::EPB + grp;
     const bool active = e_raw < m.E;
     const ElemIO io = io_from_args(m, a);
-    rhs_element<DIM, NP, NS, VC, Real, LY, CURV>(io, P, active ? e_raw : m.E - 1, active, smem, sPair,
+    rhs_element<DIM, NP, NS, VC, Real, LY, FEAT, CURV>(io, P, active ? e_raw : m.E - 1, active, smem, sPair,
                                                  sE + grp * LY::PER_ELEM, li, lane, grp);
 }
 
@@ -1529,7 +1545,7 @@ rhs_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_co
 // device memory, so a captured graph stays valid as solves are admitted and
 // retired.  Items of finished solves and items wholly inside a solve's padding
 // are skipped (uniformly over the item's lanes).
-template <int DIM, int NP, bool NS, bool VC, typename Real, int V>
+template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 __global__ void __launch_bounds__(RhsLayout<DIM, NP, NS, Real, V, VC>::THREADS, (RhsLayout<DIM, NP, NS, Real, V, VC>::MIN_BLOCKS))
 rhs_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
     using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
@@ -1570,7 +1586,7 @@ rhs_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_consta
         group_sync<LY::ITEM_THREADS>(slot);
         const int e_raw = e0 + gw;
         const bool active = e_raw < E;
-        rhs_element<DIM, NP, NS, VC, Real, LY>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT, sPair, sH, li,
+        rhs_element<DIM, NP, NS, VC, Real, LY, FEAT>(ctx->io, ctx->P, active ? e_raw : E - 1, active, sT, sPair, sH, li,
                                                lane, grp);
     }
 }
@@ -2056,7 +2072,7 @@ inline bool smem_attribute_lost(cudaError_t err, size_t bytes, std::atomic<unsig
 namespace prandtl {
 namespace {
 
-template <int DIM, int NP, bool NS, bool VC, typename Real, bool CURV>
+template <int DIM, int NP, bool NS, bool VC, typename Real, bool FEAT, bool CURV>
 cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
                           cudaStream_t s) {
     using LY = RhsLayout<DIM, NP, NS, Real, 0, VC>;
@@ -2064,9 +2080,9 @@ cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &
     const size_t sm = rhs_smem<DIM, NP, NS, VC, Real>();
     static std::atomic<unsigned> smem_set{0u};
     for (int attempt = 0; attempt < 2; ++attempt) {
-        cudaError_t err = smem_attribute_once((const void *)rhs_kernel<DIM, NP, NS, VC, Real, CURV>, (int)sm, smem_set);
+        cudaError_t err = smem_attribute_once((const void *)rhs_kernel<DIM, NP, NS, VC, Real, FEAT, CURV>, (int)sm, smem_set);
         if (err != cudaSuccess) return err;
-        rhs_kernel<DIM, NP, NS, VC, Real, CURV><<<grid, LY::THREADS, sm, s>>>(m, a, P, T);
+        rhs_kernel<DIM, NP, NS, VC, Real, FEAT, CURV><<<grid, LY::THREADS, sm, s>>>(m, a, P, T);
         err = cudaGetLastError();
         if (!smem_attribute_lost(err, sm, smem_set)) return err;
     }
@@ -2081,14 +2097,15 @@ template <int DIM, int NP, bool NS, bool VC, typename Real>
 cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
                            cudaStream_t s) {
     if (m.ngeo) {   // FP64, or the FP32-bulk Euler form (pair phase; no lifting)
-        if constexpr (sizeof(Real) == 8 || !NS) return rhs_launch_np<DIM, NP, NS, VC, Real, true>(m, a, P, T, s);
+        if constexpr (sizeof(Real) == 8 || !NS) return rhs_launch_np<DIM, NP, NS, VC, Real, true, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
     }
     if constexpr (line_form<NS, VC, Real>()) {   // by lines, but for the axisymmetric form
         if (DIM == 3 || NS || !m.rad) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
     }
     if constexpr (sizeof(Real) == 4 || (NS && !VC) || (DIM == 2 && !NS))
-        return rhs_launch_np<DIM, NP, NS, VC, Real, false>(m, a, P, T, s);
+        return P.blending || m.bcs ? rhs_launch_np<DIM, NP, NS, VC, Real, true, false>(m, a, P, T, s)
+                                   : rhs_launch_np<DIM, NP, NS, VC, Real, false, false>(m, a, P, T, s);
     else return cudaErrorNotSupported;
 }
 template <int DIM, int NP, typename Out, bool VC, bool CURV>
@@ -2114,8 +2131,9 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
         if constexpr (sizeof(Out) == 8) return lift_launch_np<DIM, NP, Out, VC, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
     }
-    if constexpr (line_form<true, VC, Out>())
-        return m.bcs ? lift_line_launch<DIM, NP, true>(m, a, P, T, s) : lift_line_launch<DIM, NP, false>(m, a, P, T, s);
+    if constexpr (VC)
+        return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)
+                     : lift_line_launch<DIM, NP, false, Out>(m, a, P, T, s);
     else return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
 }
 
@@ -2124,19 +2142,19 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
 template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_prepare_np(BatchKernelInfo *info) {
     if constexpr (line_form<NS, VC, Real>()) {
-        using L = LineShape<DIM, NP>;
+        using L = RhsLineShape<DIM, NP>;
         return line_batch_prepare<L>((const void *)rhs_line_batch_kernel<DIM, NP, NS, FEAT, V>, line_batch_smem<L>(), info);
     } else {
     using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
     const size_t sm = rhs_batch_smem<DIM, NP, NS, VC, Real, V>();
-    cudaError_t err = cudaFuncSetAttribute(rhs_batch_kernel<DIM, NP, NS, VC, Real, V>,
+    cudaError_t err = cudaFuncSetAttribute(rhs_batch_kernel<DIM, NP, NS, VC, Real, V, FEAT>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (err != cudaSuccess) return err;
     int nb = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rhs_batch_kernel<DIM, NP, NS, VC, Real, V>, LY::THREADS, sm);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rhs_batch_kernel<DIM, NP, NS, VC, Real, V, FEAT>, LY::THREADS, sm);
     if (err != cudaSuccess) return err;
     cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, rhs_batch_kernel<DIM, NP, NS, VC, Real, V>);
+    cudaFuncGetAttributes(&fa, rhs_batch_kernel<DIM, NP, NS, VC, Real, V, FEAT>);
     info->blocks_per_sm = nb;
     info->threads = LY::THREADS;
     info->smem = (int)sm;
@@ -2149,20 +2167,20 @@ template <int DIM, int NP, bool NS, bool VC, typename Real, int V, bool FEAT>
 cudaError_t rhs_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
                                 cudaStream_t s) {
     if constexpr (line_form<NS, VC, Real>()) {
-        using L = LineShape<DIM, NP>;
+        using L = RhsLineShape<DIM, NP>;
         rhs_line_batch_kernel<DIM, NP, NS, FEAT, V><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, T);
         return cudaGetLastError();
     } else {
         using LY = RhsLayout<DIM, NP, NS, Real, V, VC>;
-        rhs_batch_kernel<DIM, NP, NS, VC, Real, V><<<grid, LY::THREADS, rhs_batch_smem<DIM, NP, NS, VC, Real, V>(), s>>>(c, st, T);
+        rhs_batch_kernel<DIM, NP, NS, VC, Real, V, FEAT><<<grid, LY::THREADS, rhs_batch_smem<DIM, NP, NS, VC, Real, V>(), s>>>(c, st, T);
         return cudaGetLastError();
     }
 }
-template <int DIM, int NP, typename Out, bool VC>
+template <int DIM, int NP, typename Out, bool VC, bool FEAT>
 cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
-    if constexpr (line_form<true, VC, Out>()) {
-        using L = LiftLineShape<DIM, NP>;
-        return line_batch_prepare<L>((const void *)lift_line_batch_kernel<DIM, NP>, line_batch_smem<L>(), info);
+    if constexpr (VC) {
+        using L = LiftLineShape<DIM, NP, Out>;
+        return line_batch_prepare<L>((const void *)lift_line_batch_kernel<DIM, NP, FEAT, Out>, line_batch_smem<L>(), info);
     } else {
     using S = LiftBatchShape<DIM, NP, Out>;
     const size_t sm = lift_batch_smem<DIM, NP, Out>();
@@ -2182,12 +2200,12 @@ cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
     return cudaSuccess;
     }
 }
-template <int DIM, int NP, typename Out, bool VC>
+template <int DIM, int NP, typename Out, bool VC, bool FEAT>
 cudaError_t lift_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
                                  cudaStream_t s) {
-    if constexpr (line_form<true, VC, Out>()) {
-        using L = LiftLineShape<DIM, NP>;
-        lift_line_batch_kernel<DIM, NP><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, T);
+    if constexpr (VC) {
+        using L = LiftLineShape<DIM, NP, Out>;
+        lift_line_batch_kernel<DIM, NP, FEAT, Out><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, line_d<NP, Out>(T), T.w[0]);
     } else {
         using S = LiftBatchShape<DIM, NP, Out>;
         lift_batch_kernel<DIM, NP, Out, VC><<<grid, S::THREADS, lift_batch_smem<DIM, NP, Out>(), s>>>(c, st, T);
@@ -2240,13 +2258,15 @@ cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const 
     }()))
 }
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_prepare(int order, BatchKernelInfo *info) {
-    PRANDTL_ORDER_SWITCH((lift_batch_prepare_np<DIM, NP, Out, VC>(info)))
+cudaError_t lift_batch_prepare(int order, bool feat, BatchKernelInfo *info) {
+    PRANDTL_ORDER_SWITCH((feat ? lift_batch_prepare_np<DIM, NP, Out, VC, true>(info)
+                               : lift_batch_prepare_np<DIM, NP, Out, VC, false>(info)))
 }
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_launch(int order, int grid, const BatchClassDev &c, const BatchStage &st,
+cudaError_t lift_batch_launch(int order, bool feat, int grid, const BatchClassDev &c, const BatchStage &st,
                               const OpTables &T, cudaStream_t s) {
-    PRANDTL_ORDER_SWITCH((lift_batch_launch_np<DIM, NP, Out, VC>(grid, c, st, T, s)))
+    PRANDTL_ORDER_SWITCH((feat ? lift_batch_launch_np<DIM, NP, Out, VC, true>(grid, c, st, T, s)
+                               : lift_batch_launch_np<DIM, NP, Out, VC, false>(grid, c, st, T, s)))
 }
 
 // One translation unit per (DIM, Real, physics) instantiates its share.
@@ -2259,8 +2279,8 @@ cudaError_t lift_batch_launch(int order, int grid, const BatchClassDev &c, const
 #define PRANDTL_INSTANTIATE_LIFT(DIMV, OUT, VCV)                                                        \
     template cudaError_t lift_dispatch<DIMV, OUT, VCV>(int, const MeshDev &, const LiftArgs &,          \
                                                        const PhysParams &, const OpTables &, cudaStream_t); \
-    template cudaError_t lift_batch_prepare<DIMV, OUT, VCV>(int, BatchKernelInfo *);                    \
-    template cudaError_t lift_batch_launch<DIMV, OUT, VCV>(int, int, const BatchClassDev &, const BatchStage &, \
+    template cudaError_t lift_batch_prepare<DIMV, OUT, VCV>(int, bool, BatchKernelInfo *);                    \
+    template cudaError_t lift_batch_launch<DIMV, OUT, VCV>(int, bool, int, const BatchClassDev &, const BatchStage &, \
                                                            const OpTables &, cudaStream_t);
 
 }   // namespace prandtl

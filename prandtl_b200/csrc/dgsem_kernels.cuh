@@ -126,10 +126,10 @@ bool order_supported(int dim, int order);
 int batch_num_variants();
 cudaError_t batch_prepare_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat,
                               BatchKernelInfo *info);
-cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, BatchKernelInfo *info);
+cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, bool feat, BatchKernelInfo *info);
 cudaError_t batch_launch_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat, int grid,
                              const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s);
-cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, int grid, const BatchClassDev &c,
+cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, bool feat, int grid, const BatchClassDev &c,
                               const BatchStage &st, const OpTables &T, cudaStream_t s);
 // End of a batch step: every live solve with steps left advances its counters,
 // flips its LSRK parity, (cfl > 0) takes its next dt from lambda, and writes
@@ -171,9 +171,9 @@ template <int DIM, typename Real, bool NS, bool VC>
 cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const BatchClassDev &c,
                              const BatchStage &st, const OpTables &T, cudaStream_t s);
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_prepare(int order, BatchKernelInfo *info);
+cudaError_t lift_batch_prepare(int order, bool feat, BatchKernelInfo *info);
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_launch(int order, int grid, const BatchClassDev &c, const BatchStage &st,
+cudaError_t lift_batch_launch(int order, bool feat, int grid, const BatchClassDev &c, const BatchStage &st,
                               const OpTables &T, cudaStream_t s);
 
 // The Navier-Stokes form used for a configuration: contravariant viscous

@@ -35,29 +35,40 @@ namespace {
 // lanes of an 8-byte access on distinct banks for the lines of every direction
 // (found by enumeration: 3D Np = 4 takes 2.7 wavefronts per access against 6
 // without padding).
-template <int DIM, int NP>
+template <int DIM, int NP, typename W = double>
 struct LineShape {
+    static constexpr bool F64 = sizeof(W) == 8;
     static constexpr int ND = ipow(NP, DIM), NL = ND / NP, NF = DIM + 2;
-    static constexpr int SY = DIM == 2 ? NP + 1 : NP;
-    static constexpr int SZ = DIM == 2 ? 0 : (NP == 2 ? 5 : NP == 3 ? 9 : NP == 4 ? 19 : NP == 5 ? 25 : 39);
+    static constexpr int SY = DIM == 2 ? (F64 || NP % 2 == 0 ? NP + 1 : NP) : NP;
+    static constexpr int SZ = DIM == 2 ? 0 : (NP == 2 ? 5 : NP == 3 ? 9 : NP == 4 ? (F64 ? 19 : 16) : NP == 5 ? 25 : (F64 ? 39 : 36));
     static constexpr int ROW = (NP - 1) * (1 + SY + SZ) + 1;
-    // field rows: rho, v, beta (the two-point fluxes), then 1/beta and |v| + c (surface fluxes)
-    static constexpr int RHO = 0, V = 1, BETA = 1 + DIM, RBETA = 2 + DIM, LAM = 3 + DIM, K = 4 + DIM;
-    static constexpr int NQ = 2 + DIM;                  // rows the two-point fluxes read
-    // element constants after the rows: the neighbour table (2 DIM entries of
-    // two int2), the faces' normals and their lengths, adj(J) and det J
-    static constexpr int NBR = (K + NF) * ROW, NOR = NBR + 4 * DIM, GEO = NOR + 2 * DIM * (DIM + 1);
-    static constexpr int END = GEO + DIM * DIM + 1;
-    // element stride modulo 16 doubles that spreads a half-warp's elements over the banks
-    static constexpr int STRIDE16 = DIM == 2 ? (NP == 2 ? 2 : NP == 3 ? 3 : NP == 4 ? 4 : NP == 5 ? 5 : 10)
-                                             : (NP == 2 ? 12 : NP == 3 ? 11 : NP == 4 ? 12 : NP == 5 ? 13 : 4);
-    static constexpr int PER_ELEM = END + (STRIDE16 + 16 - END % 16) % 16;
+    // element stride, modulo the 16 double / 32 float banks, that spreads a
+    // half-warp's / warp's elements over the banks
+    static constexpr int BANKS = F64 ? 16 : 32, BYTES = sizeof(W);
+    static constexpr int STRIDE = F64 ? (DIM == 2 ? (NP == 2 ? 2 : NP == 3 ? 3 : NP == 4 ? 4 : NP == 5 ? 5 : 10)
+                                                  : (NP == 2 ? 12 : NP == 3 ? 11 : NP == 4 ? 12 : NP == 5 ? 13 : 4))
+                                      : (DIM == 2 ? (NP == 2 ? 10 : NP == 3 ? 9 : NP == 4 ? 28 : NP == 5 ? 8 : 10)
+                                                  : (NP == 2 ? 12 : NP == 3 ? 27 : NP == 4 ? 5 : NP == 5 ? 25 : 9));
+    static constexpr int padded(int end) { return end + (STRIDE + BANKS - end % BANKS) % BANKS; }
     static constexpr int EPW = NL <= 32 ? 32 / NL : 0;
     static constexpr bool WARP = EPW * NL >= 30;
     // threads per CTA when elements are packed into the CTA: 125 of 128 lanes at
     // 3D Np = 5, 126 at Np = 3, 252 of 256 at Np = 6
     static constexpr int THREADS = (!WARP && NL > 32) ? 256 : 128;
     static constexpr int EPB = WARP ? (THREADS / 32) * EPW : THREADS / NL;
+};
+// The right-hand side's shared area of an element.
+template <int DIM, int NP>
+struct RhsLineShape : LineShape<DIM, NP> {
+    using L = LineShape<DIM, NP>;
+    // field rows: rho, v, beta (the two-point fluxes), then 1/beta and |v| + c (surface fluxes)
+    static constexpr int RHO = 0, V = 1, BETA = 1 + DIM, RBETA = 2 + DIM, LAM = 3 + DIM, K = 4 + DIM;
+    static constexpr int NQ = 2 + DIM;                  // rows the two-point fluxes read
+    // then the directions' running sums, and the element's constants: the neighbour
+    // table (2 DIM entries of two int2), the faces' normals and their lengths,
+    // adj(J) and det J
+    static constexpr int NBR = (K + L::NF) * L::ROW, NOR = NBR + 4 * DIM, GEO = NOR + 2 * DIM * (DIM + 1);
+    static constexpr int PER_ELEM = L::padded(GEO + DIM * DIM + 1);
 };
 
 // Resident CTAs the register budget is sized for: 168 registers a thread.  A
@@ -72,6 +83,14 @@ template <int DIM, int NP, bool NS, int V = 0>
 constexpr int line_min_blocks() {
     return cmax(1, 65536 / ((V == 1 || (V == 0 && NS && DIM == 3 && NP == 5) ? 255 : V == 2 ? 128 : 168) *
                             LineShape<DIM, NP>::THREADS));
+}
+
+// The FP32-bulk kernels: 96 registers up to Np = 4, 128 beyond (ensemble N=2 and
+// N=4 lifts 48 and 284 us at 96, 51 and 230 us at 128; 80 is slower everywhere).
+template <int DIM, int NP, typename W>
+constexpr int lift_line_min_blocks() {
+    return sizeof(W) == 8 ? line_min_blocks<DIM, NP, false>()
+                          : cmax(1, 65536 / ((NP <= 4 ? 96 : 128) * LineShape<DIM, NP, W>::THREADS));
 }
 
 // Logarithmic mean of x, y > 0 in the form q = (x+y) / (2 mean), with
@@ -346,7 +365,7 @@ __device__ __forceinline__ void line_boundary(const ElemIO &a, const PhysParams 
 template <int DIM, int NP, bool NS, bool BLEND, bool BC, typename Sync>
 __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysParams &P, const OpTables &T, int e, bool ok,
                                                  double *sH, int ln, const Sync &sync) {
-    using L = LineShape<DIM, NP>;
+    using L = RhsLineShape<DIM, NP>;
     constexpr int ND = L::ND, NL = L::NL, NF = L::NF, ROW = L::ROW, NQ = L::NQ;
     double *sA = sH + L::K * ROW;   // the directions' running sums [NF][ROW]
     const long long Ndof = a.Ndof, e0 = (long long)e * ND;
@@ -688,14 +707,21 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
 // logarithms, left half of the threads idle on every second face item and read
 // every node's variables 3 Np times; it was bound by latency and barriers at
 // 19 warps per SM.  Measured: 32^3 Np = 4 179 -> 109 us (HBM floor 43 us for
-// 285 MB), 20^3 Np = 5 90 -> 65 us, 2D 120x60 Np = 5 unchanged at 17 us.
-template <int DIM, int NP>
-struct LiftLineShape : LineShape<DIM, NP> {
-    using L = LineShape<DIM, NP>;
+// 285 MB), 20^3 Np = 5 90 -> 65 us, 2D 120x60 Np = 5 unchanged at 17 us; in the
+// FP32-bulk form, the classes of a 96-member ensemble, 91 -> 48 us (Np = 3),
+// 123 -> 70 us (4), 363 -> 231 us (5) and 316 -> 261 us (6).
+template <int DIM, int NP, typename W>
+struct LiftLineShape : LineShape<DIM, NP, W> {
+    using L = LineShape<DIM, NP, W>;
     // rows: entropy variables [NF], derivatives along the first DIM-1 directions [DIM-1][NF];
-    // then the neighbour table and the geometry
-    static constexpr int NBR = DIM * L::NF * L::ROW, GEO = NBR + 2 * DIM, END = GEO + DIM * DIM + 1;
-    static constexpr int PER_ELEM = END + (L::STRIDE16 + 16 - END % 16) % 16;
+    // then the neighbour table (two ints a face), adj(J) and 1 / det J
+    static constexpr int NBR = DIM * L::NF * L::ROW, GEO = NBR + 4 * DIM * 4 / (int)sizeof(W);
+    static constexpr int PER_ELEM = L::padded(GEO + DIM * DIM + 1);
+};
+// D(i, l) in the working precision.
+template <typename W>
+struct LineD {
+    W d[36];
 };
 
 // ln(x / x0) for x, x0 > 0.
@@ -742,6 +768,11 @@ __device__ __forceinline__ void line_entropy(const double *s, const PhysParams &
     for (int d = 0; d < DIM; ++d) v[1 + d] = beta * vel[d];
     v[1 + DIM] = R.beta - beta;
 }
+// FP32-bulk form: the same with the logarithms of FP64-formed ratios in FP32.
+template <int DIM>
+__device__ __forceinline__ void line_entropy(const double *s, const PhysParams &P, const EntropyRef &R, float *v) {
+    conserv2entropy_rel<DIM>(s, P, R, v);
+}
 // The lifting's boundary value minus the inner trace's, as boundary_lift_trace
 // defines it (fixed mode): 1/2 (v(outer) - v1), at the no-slip walls v_wall - v1.
 template <int DIM>
@@ -770,17 +801,18 @@ __device__ __noinline__ void line_lift_boundary(const BcDev &bc, const PhysParam
     for (int f = 0; f < NF; ++f) lf[f] = 0.5 * (v2[f] - v1[f]);
 }
 
-template <int DIM, int NP, bool BC, typename Sync>
-__device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysParams &P, const OpTables &T, int e, bool ok,
-                                                  double *sV, int ln, const Sync &sync) {
-    using L = LiftLineShape<DIM, NP>;
+template <int DIM, int NP, bool BC, typename W, typename Sync>
+__device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysParams &P, const LineD<W> &T, double w0, int e,
+                                                  bool ok, W *sV, int ln, const Sync &sync) {
+    using L = LiftLineShape<DIM, NP, W>;
     constexpr int ND = L::ND, NL = L::NL, NF = L::NF, ROW = L::ROW;
-    double *sG = sV + NF * ROW, *sGeo = sV + L::GEO;
-    int2 *sNbr = reinterpret_cast<int2 *>(sV + L::NBR);   // {element, local face}
+    constexpr bool F64 = sizeof(W) == 8;
+    W *sG = sV + NF * ROW, *sGeo = sV + L::GEO;
+    int *sNbr = reinterpret_cast<int *>(sV + L::NBR);
     const long long Ndof = a.Ndof, e0 = (long long)e * ND;
     const int own0 = ln % NP + L::SY * (DIM == 2 ? 0 : ln / NP);
     constexpr int own_st = DIM == 2 ? L::SY : L::SZ;
-    LineRef R{};
+    std::conditional_t<F64, LineRef, EntropyRef> R{};
     if (ok) {
         constexpr int NG = (DIM * DIM + NL) / NL, NB = (2 * DIM + NL - 1) / NL;
         int4 nb[NB];
@@ -798,15 +830,18 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
         for (int k = 0; k < NG; ++k) g[k] = __ldg(a.geo + (long long)e * (DIM * DIM + 1) + min(ln + k * NL, DIM * DIM));
 #pragma unroll
         for (int k = 0; k < NB; ++k)
-            if (ln + k * NL < 2 * DIM)   // .y: local face, or ~(boundary condition) beside the face id
-                sNbr[ln + k * NL] = nb[k].x >= 0 ? make_int2(nb[k].x, nb[k].y) : make_int2(nb[k].z, ~nb[k].y);
+            if (ln + k * NL < 2 * DIM) {   // element and its local face, or face id and ~(boundary condition)
+                sNbr[2 * (ln + k * NL)] = nb[k].x >= 0 ? nb[k].x : nb[k].z;
+                sNbr[2 * (ln + k * NL) + 1] = nb[k].x >= 0 ? nb[k].y : ~nb[k].y;
+            }
 #pragma unroll
         for (int k = 0; k < NG; ++k)
-            if (ln + k * NL < DIM * DIM + 1) sGeo[ln + k * NL] = g[k];
-        R = line_ref<DIM>(s0, P);
+            if (ln + k * NL < DIM * DIM + 1) sGeo[ln + k * NL] = W(ln + k * NL < DIM * DIM ? g[k] : rcp(g[k]));
+        if constexpr (F64) R = line_ref<DIM>(s0, P);
+        else R = entropy_ref<DIM>(s0, P);
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-            double v[NF];
+            W v[NF];
             line_entropy<DIM>(s[i], P, R, v);
 #pragma unroll
             for (int f = 0; f < NF; ++f) sV[f * ROW + own0 + i * own_st] = v[f];
@@ -814,8 +849,8 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
     }
     sync();
 
-    const double hw0 = 0.5 / T.w[0];
-    double gl[NP][NF];
+    const W hw0 = W(0.5 / w0);
+    W gl[NP][NF];
 #pragma unroll 1
     for (int dir = 0; dir < DIM; ++dir) {
         if (ok) {
@@ -828,7 +863,7 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
             int2 nb[2];
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
-                nb[side] = sNbr[2 * dir + side];
+                nb[side] = make_int2(sNbr[2 * (2 * dir + side)], sNbr[2 * (2 * dir + side) + 1]);
                 long long g = e0 + ga * (ln % NP) + gb * (ln / NP) + side * (NP - 1) * gt;
                 if (!BC || nb[side].y >= 0) {
                     int na, nbs, nt;
@@ -839,16 +874,16 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
                 for (int f = 0; f < NF; ++f) s[side][f] = ldg_now(a.u + f * Ndof + g);
             }
             // derivative along the line: sum_l D(i, l) v_l
-            double v0[NF], v1[NF];
+            W v0[NF], v1[NF];
 #pragma unroll
             for (int l = 0; l < NP; ++l) {
-                double v[NF];
+                W v[NF];
 #pragma unroll
                 for (int f = 0; f < NF; ++f) v[f] = sV[f * ROW + n0 + l * st];
 #pragma unroll
                 for (int i = 0; i < NP; ++i)
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) gl[i][f] = l == 0 ? T.D[i * NP] * v[f] : fma(T.D[i * NP + l], v[f], gl[i][f]);
+                    for (int f = 0; f < NF; ++f) gl[i][f] = l == 0 ? T.d[i * NP] * v[f] : fma(T.d[i * NP + l], v[f], gl[i][f]);
                 if (l == 0)
 #pragma unroll
                     for (int f = 0; f < NF; ++f) v0[f] = v[f];
@@ -861,7 +896,7 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
             // adj(J), so the jump adds to the derivative along that row's direction
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
-                double vn[NF], jump[NF];
+                W vn[NF], jump[NF];
                 if (BC && nb[side].y < 0) {
                     double in[NF], nor[DIM], lf[NF];
 #pragma unroll
@@ -870,7 +905,7 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
                     for (int d = 0; d < DIM; ++d) nor[d] = __ldg(a.fnor + (long long)nb[side].x * DIM + d);
                     line_lift_boundary<DIM>(a.bcs[~nb[side].y], P, in, nor, lf);
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) jump[f] = 2.0 * lf[f];
+                    for (int f = 0; f < NF; ++f) jump[f] = W(2.0 * lf[f]);
                 } else {
                     line_entropy<DIM>(s[side], P, R, vn);
 #pragma unroll
@@ -883,7 +918,7 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
                 }
             }
             if (dir < DIM - 1) {
-                double *out = sG + dir * NF * ROW + n0;
+                W *out = sG + dir * NF * ROW + n0;
 #pragma unroll
                 for (int i = 0; i < NP; ++i)
 #pragma unroll
@@ -896,9 +931,9 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
 
     // ---- node by node: gradients (grad1 adj / J, LiftingBR1.cpp:205-206), the chain rule
     // and the contravariant viscous flux adj Fv^T, rows f = 1..NF-1, in line order
-    const double mJ = rcp(sGeo[DIM * DIM]);
-    double *gout = reinterpret_cast<double *>(a.grad) + (long long)e * (DIM * (NF - 1) * ND);
-    double adj[DIM][DIM];
+    const W mJ = sGeo[DIM * DIM];
+    W *gout = reinterpret_cast<W *>(a.grad) + (long long)e * (DIM * (NF - 1) * ND);
+    W adj[DIM][DIM];
 #pragma unroll
     for (int r = 0; r < DIM; ++r)
 #pragma unroll
@@ -906,9 +941,13 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const int n = own0 + i * own_st;
-        double s[NF], g1[DIM][NF], g[DIM][NF], vel[DIM], Vc[DIM][NF];
+        double s[NF];
+        W sw[NF], g1[DIM][NF], g[DIM][NF], vel[DIM], Vc[DIM][NF];
 #pragma unroll
-        for (int f = 0; f < NF; ++f) s[f] = __ldg(a.u + f * Ndof + e0 + ln + NL * i);
+        for (int f = 0; f < NF; ++f) {
+            s[f] = __ldg(a.u + f * Ndof + e0 + ln + NL * i);
+            sw[f] = W(s[f]);
+        }
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
 #pragma unroll
@@ -919,33 +958,34 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
         for (int q = 0; q < DIM; ++q) {
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
-                double x = g1[0][f] * adj[0][q];
+                W x = g1[0][f] * adj[0][q];
 #pragma unroll
                 for (int r = 1; r < DIM; ++r) x = fma(g1[r][f], adj[r][q], x);
                 g[q][f] = x * mJ;
             }
-            entropygrad2primgrad<DIM, double>(s, P, g[q]);
+            entropygrad2primgrad<DIM, W>(sw, P, g[q]);
         }
+        // the node's velocity and pressure, formed in FP64
         const double rr = rcp(s[0]);
         double vv = 0.0;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
-            vel[d] = s[1 + d] * rr;
-            vv += vel[d] * vel[d];
+            vel[d] = W(s[1 + d] * rr);
+            vv = fma(s[1 + d], s[1 + d], vv);
         }
-        const double p = P.gammaM1 * (s[NF - 1] - s[0] * (0.5 * vv));
+        const double p = P.gammaM1 * fma(-0.5 * rr, vv, s[NF - 1]);
 #pragma unroll
         for (int r = 0; r < DIM; ++r)
 #pragma unroll
-            for (int f = 0; f < NF; ++f) Vc[r][f] = 0.0;
-        viscous_flux<DIM, double>(s[0], rr, vel, p, g, P, [&](int f, int cc, double val) {
+            for (int f = 0; f < NF; ++f) Vc[r][f] = 0;
+        viscous_flux<DIM, W>(sw[0], W(rr), vel, W(p), g, P, [&](int f, int cc, W val) {
 #pragma unroll
             for (int r = 0; r < DIM; ++r) Vc[r][f] = fma(adj[r][cc], val, Vc[r][f]);
         });
         const int c[3] = {ln % NP, DIM == 2 ? i : ln / NP, i};
 #pragma unroll
         for (int r = 0; r < DIM; ++r) {
-            double *out = gout + r * (NF - 1) * ND + c[r] * NL + line_index<DIM, NP>(r, c);
+            W *out = gout + r * (NF - 1) * ND + c[r] * NL + line_index<DIM, NP>(r, c);
 #pragma unroll
             for (int f = 1; f < NF; ++f) out[(f - 1) * ND] = Vc[r][f];
         }
@@ -980,7 +1020,7 @@ struct LineSync {
 template <int DIM, int NP, bool NS, bool BLEND, bool BC>
 __global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, NS>()))
 rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
-    using L = LineShape<DIM, NP>;
+    using L = RhsLineShape<DIM, NP>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const LineLane<L> q;
     const bool ok = q.lane_ok && q.e < m.E;
@@ -988,19 +1028,20 @@ rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __gr
     const ElemIO io = io_from_args(m, a);
     rhs_line_element<DIM, NP, NS, BLEND, BC>(io, P, T, ok ? q.e : 0, ok, sH, q.ln, LineSync<L>{});
 }
-template <int DIM, int NP, bool BC>
-__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, false>()))
-lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
-    using L = LiftLineShape<DIM, NP>;
+template <int DIM, int NP, bool BC, typename W>
+__global__ void __launch_bounds__(LineShape<DIM, NP, W>::THREADS, (lift_line_min_blocks<DIM, NP, W>()))
+lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_constant__ LineD<W> T, double w0) {
+    using L = LiftLineShape<DIM, NP, W>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const LineLane<L> q;
     const bool ok = q.lane_ok && q.e < m.E;
-    double *sV = reinterpret_cast<double *>(smem_raw) + q.el * L::PER_ELEM;
+    W *sV = reinterpret_cast<W *>(smem_raw) + q.el * L::PER_ELEM;
     RhsArgs r{};
     r.u = a.u;
     r.grad = a.grad;
+    r.grad32 = a.grad32;
     const ElemIO io = io_from_args(m, r);
-    lift_line_element<DIM, NP, BC>(io, P, T, ok ? q.e : 0, ok, sV, q.ln, LineSync<L>{});
+    lift_line_element<DIM, NP, BC, W>(io, P, T, w0, ok ? q.e : 0, ok, sV, q.ln, LineSync<L>{});
 }
 
 // Persistent batch kernel: a fixed grid walks the class's work items, each the
@@ -1008,7 +1049,7 @@ lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __
 // solve's element range is padded to BATCH_CHUNK in the class prefix; every
 // chunk holds ceil(BATCH_CHUNK / EPI) items, the last one shorter.  FEAT: the
 // class's solves have blending or boundary conditions.
-template <typename L, typename Element>
+template <typename L, typename W, typename Element>
 __device__ __forceinline__ void line_batch_items(const BatchClassDev &c, const BatchStage &st, const Element &element) {
     constexpr int EPI = L::WARP ? L::EPW : L::EPB;                 // elements per item
     constexpr int IPC = (BATCH_CHUNK + EPI - 1) / EPI;             // items per chunk
@@ -1019,7 +1060,7 @@ __device__ __forceinline__ void line_batch_items(const BatchClassDev &c, const B
     WarpCtx *ctx = reinterpret_cast<WarpCtx *>(smem_raw) + slot;
     const int el = il / L::NL, ln = il - el * L::NL;
     const bool lane_ok = el < EPI;
-    double *sH = reinterpret_cast<double *>(smem_raw + CTX_RESERVE) + (slot * EPI + (lane_ok ? el : 0)) * L::PER_ELEM;
+    W *sH = reinterpret_cast<W *>(smem_raw + CTX_RESERVE) + (slot * EPI + (lane_ok ? el : 0)) * L::PER_ELEM;
     const LineSync<L> sync{};
     const int n = c.hdr[0];
     const int total = n > 0 ? c.prefix[n] / BATCH_CHUNK * IPC : 0;
@@ -1046,21 +1087,19 @@ __device__ __forceinline__ void line_batch_items(const BatchClassDev &c, const B
 template <int DIM, int NP, bool NS, bool FEAT, int V>
 __global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, NS, V>()))
 rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
-    using L = LineShape<DIM, NP>;
-    line_batch_items<L>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sH, int ln,
+    using L = RhsLineShape<DIM, NP>;
+    line_batch_items<L, double>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sH, int ln,
                                    const LineSync<L> &sync) {
         rhs_line_element<DIM, NP, NS, FEAT, FEAT>(io, P, T, e, ok, sH, ln, sync);
     });
 }
-// (the lifting's boundary code is compiled into every batch kernel: one class
-// launch serves solves with and without boundary conditions)
-template <int DIM, int NP>
-__global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, false>()))
-lift_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ OpTables T) {
-    using L = LiftLineShape<DIM, NP>;
-    line_batch_items<L>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sV, int ln,
-                                   const LineSync<L> &sync) {
-        lift_line_element<DIM, NP, true>(io, P, T, e, ok, sV, ln, sync);
+template <int DIM, int NP, bool FEAT, typename W>
+__global__ void __launch_bounds__(LineShape<DIM, NP, W>::THREADS, (lift_line_min_blocks<DIM, NP, W>()))
+lift_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_constant__ LineD<W> T, double w0) {
+    using L = LiftLineShape<DIM, NP, W>;
+    line_batch_items<L, W>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, W *sV, int ln,
+                                      const LineSync<L> &sync) {
+        lift_line_element<DIM, NP, FEAT, W>(io, P, T, w0, e, ok, sV, ln, sync);
     });
 }
 template <typename L>
@@ -1080,19 +1119,18 @@ cudaError_t line_batch_prepare(const void *k, size_t smem, BatchKernelInfo *info
     return cudaSuccess;
 }
 template <typename L>
-constexpr size_t line_batch_smem() { return CTX_RESERVE + sizeof(double) * (size_t)L::EPB * L::PER_ELEM; }
-template <typename L, typename Kernel, typename Args>
-cudaError_t line_launch(Kernel k, std::atomic<unsigned> &smem_set, const MeshDev &m, const Args &a, const PhysParams &P,
-                        const OpTables &T, cudaStream_t s) {
+constexpr size_t line_batch_smem() { return CTX_RESERVE + (size_t)L::BYTES * L::EPB * L::PER_ELEM; }
+template <typename L, typename Kernel, typename... Args>
+cudaError_t line_launch(Kernel k, std::atomic<unsigned> &smem_set, cudaStream_t s, const MeshDev &m, const Args &...args) {
     int threads = L::THREADS;
     if constexpr (L::WARP)   // small meshes: one-warp CTAs, so that every SM gets work
         while (threads > 32 && m.E < 148 * (threads / 32) * L::EPW) threads /= 2;
     const int epb = L::WARP ? threads / 32 * L::EPW : L::EPB;
-    const size_t sm = sizeof(double) * (size_t)epb * L::PER_ELEM;
+    const size_t sm = (size_t)L::BYTES * epb * L::PER_ELEM;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        cudaError_t err = smem_attribute_once((const void *)k, (int)sizeof(double) * L::EPB * L::PER_ELEM, smem_set);
+        cudaError_t err = smem_attribute_once((const void *)k, L::BYTES * L::EPB * L::PER_ELEM, smem_set);
         if (err != cudaSuccess) return err;
-        k<<<(m.E + epb - 1) / epb, threads, sm, s>>>(m, a, P, T);
+        k<<<(m.E + epb - 1) / epb, threads, sm, s>>>(m, args...);
         err = cudaGetLastError();
         if (!smem_attribute_lost(err, sm, smem_set)) return err;
     }
@@ -1101,12 +1139,18 @@ cudaError_t line_launch(Kernel k, std::atomic<unsigned> &smem_set, const MeshDev
 template <int DIM, int NP, bool NS, bool BLEND, bool BC>
 cudaError_t rhs_line_launch(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
     static std::atomic<unsigned> smem_set{0u};
-    return line_launch<LineShape<DIM, NP>>(rhs_line_kernel<DIM, NP, NS, BLEND, BC>, smem_set, m, a, P, T, s);
+    return line_launch<RhsLineShape<DIM, NP>>(rhs_line_kernel<DIM, NP, NS, BLEND, BC>, smem_set, s, m, a, P, T);
 }
-template <int DIM, int NP, bool BC>
+template <int NP, typename W>
+LineD<W> line_d(const OpTables &T) {
+    LineD<W> D{};
+    for (int q = 0; q < NP * NP; ++q) D.d[q] = W(T.D[q]);
+    return D;
+}
+template <int DIM, int NP, bool BC, typename W>
 cudaError_t lift_line_launch(const MeshDev &m, const LiftArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
     static std::atomic<unsigned> smem_set{0u};
-    return line_launch<LiftLineShape<DIM, NP>>(lift_line_kernel<DIM, NP, BC>, smem_set, m, a, P, T, s);
+    return line_launch<LiftLineShape<DIM, NP, W>>(lift_line_kernel<DIM, NP, BC, W>, smem_set, s, m, a, P, line_d<NP, W>(T), T.w[0]);
 }
 template <int DIM, int NP, bool NS>
 cudaError_t rhs_line_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {

@@ -378,7 +378,7 @@ prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc,
     if (first_ok < 0) return bfail(b, PRANDTL_EUNSUPPORTED, "no RHS launch shape fits this device");
     c.variant = first_ok;
     if (ns) {
-        BCK(b, batch_prepare_lift(dim, order, vc, fp32, &c.linfo), "prepare batch lift kernel");
+        BCK(b, batch_prepare_lift(dim, order, vc, fp32, feat, &c.linfo), "prepare batch lift kernel");
         if (c.linfo.blocks_per_sm <= 0) return bfail(b, PRANDTL_EUNSUPPORTED, "lift kernel does not fit this device");
     }
     const size_t words = 2 * (size_t)b->cap + 5;
@@ -405,7 +405,7 @@ prandtl_status enqueue_step(prandtl_batch *b, cudaStream_t s) {
             Class &c = kv.second;
             if (c.ns) {
                 const int grid = c.linfo.blocks_per_sm * b->num_sms;
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, grid, c.dev, st, c.T, s), "batch lift launch");
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, grid, c.dev, st, c.T, s), "batch lift launch");
             }
             const int grid = c.rinfo[c.variant].blocks_per_sm * b->num_sms;
             BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, c.variant, c.feat, grid, c.dev, st, c.T, s),
@@ -441,7 +441,7 @@ prandtl_status tune_step(prandtl_batch *b, int v) {
             if (c.ns) {
                 const int grid = c.linfo.blocks_per_sm * b->num_sms;
                 BCK(b, cudaEventRecord(b->tev[q], b->stream), "event");
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, grid, c.dev, st, c.T, b->stream),
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, grid, c.dev, st, c.T, b->stream),
                     "batch lift launch");
                 BCK(b, cudaEventRecord(b->tev[q + 1], b->stream), "event");
             }
@@ -1153,10 +1153,10 @@ prandtl_status prandtl_batch_tune(prandtl_batch *b, int reps) {
         if (c.ids.empty()) continue;
         if (c.ns) {
             const int lgrid = c.linfo.blocks_per_sm * b->num_sms;
-            BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
+            BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
             BCK(b, cudaEventRecord(b->ev0, b->stream), "event");
             for (int r = 0; r < reps; ++r)
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
             BCK(b, cudaEventRecord(b->ev1, b->stream), "event");
             if ((st = bwait(b)) != PRANDTL_OK) return st;
             float lms = 0.f;

@@ -261,11 +261,12 @@ __device__ __forceinline__ void rk_epilogue(const ElemIO &a, const double (*al)[
     const bool need_b = (mode == EPI_LSRK && a.rkA != 0.0) || mode == EPI_SSP2 || mode == EPI_SSP3;
     const double *pb = mode == EPI_LSRK ? a.du : a.x0;
     const double cx = mode == EPI_SSP2 ? 3. / 4 : 1. / 3, cy = mode == EPI_SSP2 ? 1. / 4 : 2. / 3;
+    constexpr int KB = 6 * NP * NF <= 128 ? NP : (NP + 1) / 2;
 #pragma unroll
-    for (int i0 = 0; i0 < NP; i0 += 2) {
-        double ua[2][NF], ub[2][NF];
+    for (int i0 = 0; i0 < NP; i0 += KB) {
+        double ua[KB][NF], ub[KB][NF];
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+        for (int k = 0; k < KB; ++k)
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
                 const long long g = f * Ndof + node0 + (i0 + k) * step;
@@ -273,7 +274,7 @@ __device__ __forceinline__ void rk_epilogue(const ElemIO &a, const double (*al)[
                 ub[k][f] = i0 + k < NP && need_b ? pb[g] : 0.0;
             }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < KB; ++k) {
             if (i0 + k >= NP) continue;
             const long long gnode = node0 + (i0 + k) * step;
             double v[NF];

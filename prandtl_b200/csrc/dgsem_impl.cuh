@@ -2100,6 +2100,9 @@ cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams 
         if constexpr (sizeof(Real) == 8 || !NS) return rhs_launch_np<DIM, NP, NS, VC, Real, true, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
     }
+    if constexpr (sizeof(Real) == 8 && NS && !VC) {   // reference mode: plain solves by lines
+        if (m.ref_lines && !P.blending) return rhs_line_launch<DIM, NP, true, false, false, true>(m, a, P, T, s);
+    }
     if constexpr (line_form<NS, VC, Real>()) {   // by lines, but for the axisymmetric form
         if (DIM == 3 || NS || !m.rad) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
     }
@@ -2130,6 +2133,9 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
     if (m.ngeo) {
         if constexpr (sizeof(Out) == 8) return lift_launch_np<DIM, NP, Out, VC, true>(m, a, P, T, s);
         else return cudaErrorNotSupported;
+    }
+    if constexpr (sizeof(Out) == 8 && !VC) {
+        if (m.ref_lines && !P.blending) return lift_line_launch<DIM, NP, false, Out, true>(m, a, P, T, s);
     }
     if constexpr (VC)
         return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)

@@ -34,6 +34,10 @@ struct MeshDev {
     const double *ngeo;
     const double *fnn;
     const double *snor;
+    // FP64 Navier-Stokes in the reference mode: run by lines.  The mesh has no
+    // boundary conditions, its normals are the elements' adjugate rows, and the
+    // gradient buffer holds DIM (NF-1) (1 + 2/Np) values per node
+    bool ref_lines = false;
 };
 
 struct RhsArgs {

@@ -363,7 +363,13 @@ __device__ __forceinline__ void line_boundary(const ElemIO &a, const PhysParams 
 // One element of a lane group: lane `ln` of NL, `sH` the element's shared area.
 // Every thread of the synchronising group calls it; lanes without an element
 // or a line have ok = false.  SYNC orders the group's shared memory.
-template <int DIM, int NP, bool NS, bool BLEND, bool BC, typename Sync>
+// REF: Navier-Stokes in the reference mode (quirks == 0), whose viscous rows
+// come in two parts: the volume's, of the element's last node's state
+// (DGSEMIntegrator.cpp:620), and the face nodes' own (lift_line_element).  The
+// general form reads 15 gradients per node, twice per face node, and evaluates
+// viscous fluxes from them at 12 warps per SM; here 18 values per node pass
+// through memory.  20^3 Np = 4: RHS 145 -> 66 us, lifting 49 -> 40 us.
+template <int DIM, int NP, bool NS, bool BLEND, bool BC, bool REF, typename Sync>
 __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysParams &P, const OpTables &T, int e, bool ok,
                                                  double *sH, int ln, const Sync &sync) {
     using L = RhsLineShape<DIM, NP>;
@@ -371,7 +377,9 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
     double *sA = sH + L::K * ROW;   // the directions' running sums [NF][ROW]
     const long long Ndof = a.Ndof, e0 = (long long)e * ND;
     const double gamma = P.gamma, gm1 = P.gammaM1, gm1i = P.gammaM1Inverse;
-    const bool quirk3 = !NS && P.quirks == 0;   // the Navier-Stokes form here is the fixed mode
+    const bool quirk3 = REF || (!NS && P.quirks == 0);
+    static_assert(!REF || (NS && !BLEND && !BC), "the reference mode's lines are for plain Navier-Stokes solves");
+    const double *gface = reinterpret_cast<const double *>(a.grad) + Ndof * (DIM * (NF - 1));   // REF: [E][2 DIM][NF-1][NL]
     // a lane's nodes in the node-wise phases: ln, ln + NL, ... (those of its last-direction line)
     const int own0 = ln % NP + L::SY * (DIM == 2 ? 0 : ln / NP);
     constexpr int own_st = DIM == 2 ? L::SY : L::SZ;
@@ -540,6 +548,28 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
                 far = far || !(d * d < 1e-4 * (s * s));
             }
         }
+        // the reference's 3D zeta flux slot holds, for a node's lower partners, the eta flux between the
+        // partner and the last node of its eta line (:702), zero on that node itself
+        const bool eta = REF && DIM == 3 && dir == 2;
+        double qg[NP][NQ];
+        if constexpr (REF && DIM == 3) {
+#pragma unroll
+            for (int i = 0; i < NP; ++i)
+#pragma unroll
+                for (int k = 0; k < NQ; ++k) qg[i][k] = q[i][k];
+            if (ok && eta) {
+#pragma unroll
+                for (int i = 0; i < NP - 1; ++i) {
+#pragma unroll
+                    for (int k = 0; k < NQ; ++k) qg[i][k] = sH[k * ROW + ln % NP + L::SY * (NP - 1) + i * st];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const double x = q[i][k * (1 + DIM)], y = qg[i][k * (1 + DIM)], d = y - x, s = y + x;
+                        far = far || !(d * d < 1e-4 * (s * s));
+                    }
+                }
+            }
+        }
         const bool any_far = __any_sync(0xffffffffu, far);
         if (ok) {
 #pragma unroll
@@ -548,7 +578,17 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
                 for (int f = 0; f < NF; ++f) al[i][f] = 0.0;
             auto pairs = [&](auto near) {
 #pragma unroll
-                for (int i = 0; i < NP - 1; ++i)
+                for (int i = 0; i < NP - 1; ++i) {
+                    double G[NF];
+                    if constexpr (REF && DIM == 3) {
+                        if (eta) {
+                            const double mg[3] = {sGeo[3], sGeo[4], sGeo[5]};
+                            line_flux<DIM, decltype(near)::value>(q[i], qg[i], mg, gm1i, G);
+                            if (ln / NP == NP - 1)
+#pragma unroll
+                                for (int f = 0; f < NF; ++f) G[f] = 0.0;
+                        }
+                    }
 #pragma unroll
                     for (int l = i + 1; l < NP; ++l) {
                         double F[NF];
@@ -557,9 +597,10 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
                             al[i][f] = fma(-dil, F[f], al[i][f]);
-                            al[l][f] = fma(-dli, F[f], al[l][f]);
+                            al[l][f] = fma(-dli, eta ? G[f] : F[f], al[l][f]);
                         }
                     }
+                }
             };
             if (any_far) pairs(std::false_type{});
             else pairs(std::true_type{});
@@ -605,12 +646,20 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
 #pragma unroll
                 for (int f = 0; f < NF; ++f) s[side][f] = ldg_now(a.u + f * Ndof + g);
                 if constexpr (NS) {
-                    const double *gv = grad + ((long long)nb.x * DIM + dn) * ((NF - 1) * ND) + in * NL + ln;
+                    const double *gv = REF ? gface + ((long long)nb.x * (2 * DIM) + nb.y) * ((NF - 1) * NL) + ln
+                                           : grad + ((long long)nb.x * DIM + dn) * ((NF - 1) * ND) + in * NL + ln;
 #pragma unroll
-                    for (int f = 0; f < NF - 1; ++f) vn[side][f] = ldg_now(gv + f * ND);
+                    for (int f = 0; f < NF - 1; ++f) vn[side][f] = ldg_now(gv + f * (REF ? NL : ND));
                 }
             }
             double vo[2][NF - 1];   // the viscous rows of the line's end nodes
+            if constexpr (REF) {
+#pragma unroll
+                for (int side = 0; side < 2; ++side)
+#pragma unroll
+                    for (int f = 0; f < NF - 1; ++f)
+                        vo[side][f] = ldg_now(gface + (((long long)e * (2 * DIM) + 2 * dir + side) * (NF - 1) + f) * NL + ln);
+            }
             if constexpr (NS) {
                 const double *gv = grad + ((long long)e * DIM + dir) * ((NF - 1) * ND) + ln;
 #pragma unroll
@@ -624,11 +673,12 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
                     for (int i = 0; i < NP; ++i)
 #pragma unroll
                         for (int f = 1; f < NF; ++f) al[i][f] = fma(T.Dhat[i * NP + l], v[l][f - 1], al[i][f]);
+                if constexpr (!REF)
 #pragma unroll
-                for (int f = 0; f < NF - 1; ++f) {
-                    vo[0][f] = v[0][f];
-                    vo[1][f] = v[NP - 1][f];
-                }
+                    for (int f = 0; f < NF - 1; ++f) {
+                        vo[0][f] = v[0][f];
+                        vo[1][f] = v[NP - 1][f];
+                    }
             }
             // ---- the line's two faces
 #pragma unroll
@@ -645,9 +695,29 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
                     double nor[DIM], qn[L::K], qo[L::K], qa[L::K], qb[L::K], F[NF];
 #pragma unroll
                     for (int d = 0; d < DIM; ++d) nor[d] = sNor[lf * (DIM + 1) + d];
-                    line_prim<DIM>(s[side], gamma, gm1, qn);
+                    if constexpr (REF) {
+                        // Q8 (BasicOperations.cpp:33-34 via NavierStokesFlux.cpp:14): the surface flux reads
+                        // states whose momentum slots hold velocities
+                        double so[NF];
+                        const double rn = rcp(s[side][0]);
 #pragma unroll
-                    for (int k = 0; k < L::K; ++k) qo[k] = sH[k * ROW + n0 + ie * st];
+                        for (int d = 0; d < DIM; ++d) s[side][1 + d] *= rn;
+                        line_prim<DIM>(s[side], gamma, gm1, qn);
+                        double vv = 0.0;
+                        so[0] = sH[n0 + ie * st];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) {
+                            so[1 + d] = sH[(L::V + d) * ROW + n0 + ie * st];
+                            vv = fma(so[1 + d], so[1 + d], vv);
+                        }
+                        // E = p / (gamma - 1) + rho |v|^2 / 2 with p = rho / (2 beta)
+                        so[NF - 1] = 0.5 * so[0] * fma(gm1i, sH[L::RBETA * ROW + n0 + ie * st], vv);
+                        line_prim<DIM>(so, gamma, gm1, qo);
+                    } else {
+                        line_prim<DIM>(s[side], gamma, gm1, qn);
+#pragma unroll
+                        for (int k = 0; k < L::K; ++k) qo[k] = sH[k * ROW + n0 + ie * st];
+                    }
                     // both elements evaluate the face with the operands in Elem1, Elem2 order
                     const bool first = sNbr[2 * lf + 1].y == 0;
 #pragma unroll
@@ -802,7 +872,10 @@ __device__ __noinline__ void line_lift_boundary(const BcDev &bc, const PhysParam
     for (int f = 0; f < NF; ++f) lf[f] = 0.5 * (v2[f] - v1[f]);
 }
 
-template <int DIM, int NP, bool BC, typename W, typename Sync>
+// REF (reference mode): the rows of the volume term take the state of the
+// element's last node (Q1), and the face nodes' own rows follow the volume rows
+// of all elements, [E][2 DIM][NF-1][face node].
+template <int DIM, int NP, bool BC, bool REF, typename W, typename Sync>
 __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysParams &P, const LineD<W> &T, double w0, int e,
                                                   bool ok, W *sV, int ln, const Sync &sync) {
     using L = LiftLineShape<DIM, NP, W>;
@@ -939,6 +1012,21 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
     for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int q = 0; q < DIM; ++q) adj[r][q] = sGeo[r * DIM + q];
+    W last[3 + DIM];   // REF: rho, 1/rho, v, p of the element's last node
+    if constexpr (REF) {
+        double s[NF], vv = 0.0;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) s[f] = __ldg(a.u + f * Ndof + e0 + ND - 1);
+        const double rr = rcp(s[0]);
+        last[0] = s[0];
+        last[1] = rr;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            last[2 + d] = s[1 + d] * rr;
+            vv = fma(s[1 + d], s[1 + d], vv);
+        }
+        last[2 + DIM] = P.gammaM1 * fma(-0.5 * rr, vv, s[NF - 1]);
+    }
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const int n = own0 + i * own_st;
@@ -975,15 +1063,31 @@ __device__ __forceinline__ void lift_line_element(const ElemIO &a, const PhysPar
             vv = fma(s[1 + d], s[1 + d], vv);
         }
         const double p = P.gammaM1 * fma(-0.5 * rr, vv, s[NF - 1]);
+        auto rows = [&](W rho, W rrho, const W *vl, W pr) {
 #pragma unroll
-        for (int r = 0; r < DIM; ++r)
+            for (int r = 0; r < DIM; ++r)
 #pragma unroll
-            for (int f = 0; f < NF; ++f) Vc[r][f] = 0;
-        viscous_flux<DIM, W>(sw[0], W(rr), vel, W(p), g, P, [&](int f, int cc, W val) {
+                for (int f = 0; f < NF; ++f) Vc[r][f] = 0;
+            viscous_flux<DIM, W>(rho, rrho, vl, pr, g, P, [&](int f, int cc, W val) {
 #pragma unroll
-            for (int r = 0; r < DIM; ++r) Vc[r][f] = fma(adj[r][cc], val, Vc[r][f]);
-        });
+                for (int r = 0; r < DIM; ++r) Vc[r][f] = fma(adj[r][cc], val, Vc[r][f]);
+            });
+        };
+        rows(sw[0], W(rr), vel, W(p));
         const int c[3] = {ln % NP, DIM == 2 ? i : ln / NP, i};
+        if constexpr (REF) {
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) {
+                const int lf = c[r] == 0 ? 2 * r : c[r] == NP - 1 ? 2 * r + 1 : -1;
+                if (lf >= 0) {
+                    W *out = reinterpret_cast<W *>(a.grad) + Ndof * (DIM * (NF - 1)) +
+                             ((long long)e * (2 * DIM) + lf) * ((NF - 1) * NL) + face_tangential<DIM, NP>(r, c);
+#pragma unroll
+                    for (int f = 1; f < NF; ++f) out[(f - 1) * NL] = Vc[r][f];
+                }
+            }
+            rows(W(last[0]), W(last[1]), last + 2, W(last[2 + DIM]));
+        }
 #pragma unroll
         for (int r = 0; r < DIM; ++r) {
             W *out = gout + r * (NF - 1) * ND + c[r] * NL + line_index<DIM, NP>(r, c);
@@ -1018,7 +1122,7 @@ struct LineSync {
 
 // One-shot kernels.  blockDim may be any multiple of 32 up to THREADS when
 // elements are packed into warps, THREADS otherwise.
-template <int DIM, int NP, bool NS, bool BLEND, bool BC>
+template <int DIM, int NP, bool NS, bool BLEND, bool BC, bool REF>
 __global__ void __launch_bounds__(LineShape<DIM, NP>::THREADS, (line_min_blocks<DIM, NP, NS>()))
 rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __grid_constant__ OpTables T) {
     using L = RhsLineShape<DIM, NP>;
@@ -1027,9 +1131,9 @@ rhs_line_kernel(const MeshDev m, const RhsArgs a, const PhysParams P, const __gr
     const bool ok = q.lane_ok && q.e < m.E;
     double *sH = reinterpret_cast<double *>(smem_raw) + q.el * L::PER_ELEM;
     const ElemIO io = io_from_args(m, a);
-    rhs_line_element<DIM, NP, NS, BLEND, BC>(io, P, T, ok ? q.e : 0, ok, sH, q.ln, LineSync<L>{});
+    rhs_line_element<DIM, NP, NS, BLEND, BC, REF>(io, P, T, ok ? q.e : 0, ok, sH, q.ln, LineSync<L>{});
 }
-template <int DIM, int NP, bool BC, typename W>
+template <int DIM, int NP, bool BC, bool REF, typename W>
 __global__ void __launch_bounds__(LineShape<DIM, NP, W>::THREADS, (lift_line_min_blocks<DIM, NP, W>()))
 lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __grid_constant__ LineD<W> T, double w0) {
     using L = LiftLineShape<DIM, NP, W>;
@@ -1042,7 +1146,7 @@ lift_line_kernel(const MeshDev m, const LiftArgs a, const PhysParams P, const __
     r.grad = a.grad;
     r.grad32 = a.grad32;
     const ElemIO io = io_from_args(m, r);
-    lift_line_element<DIM, NP, BC, W>(io, P, T, w0, ok ? q.e : 0, ok, sV, q.ln, LineSync<L>{});
+    lift_line_element<DIM, NP, BC, REF, W>(io, P, T, w0, ok ? q.e : 0, ok, sV, q.ln, LineSync<L>{});
 }
 
 // Persistent batch kernel: a fixed grid walks the class's work items, each the
@@ -1091,7 +1195,7 @@ rhs_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_c
     using L = RhsLineShape<DIM, NP>;
     line_batch_items<L, double>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, double *sH, int ln,
                                    const LineSync<L> &sync) {
-        rhs_line_element<DIM, NP, NS, FEAT, FEAT>(io, P, T, e, ok, sH, ln, sync);
+        rhs_line_element<DIM, NP, NS, FEAT, FEAT, false>(io, P, T, e, ok, sH, ln, sync);
     });
 }
 template <int DIM, int NP, bool FEAT, typename W>
@@ -1100,7 +1204,7 @@ lift_line_batch_kernel(const BatchClassDev c, const BatchStage st, const __grid_
     using L = LiftLineShape<DIM, NP, W>;
     line_batch_items<L, W>(c, st, [&](const ElemIO &io, const PhysParams &P, int e, bool ok, W *sV, int ln,
                                       const LineSync<L> &sync) {
-        lift_line_element<DIM, NP, FEAT, W>(io, P, T, w0, e, ok, sV, ln, sync);
+        lift_line_element<DIM, NP, FEAT, false, W>(io, P, T, w0, e, ok, sV, ln, sync);
     });
 }
 template <typename L>
@@ -1137,10 +1241,10 @@ cudaError_t line_launch(Kernel k, std::atomic<unsigned> &smem_set, cudaStream_t 
     }
     return cudaErrorInvalidValue;
 }
-template <int DIM, int NP, bool NS, bool BLEND, bool BC>
+template <int DIM, int NP, bool NS, bool BLEND, bool BC, bool REF = false>
 cudaError_t rhs_line_launch(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
     static std::atomic<unsigned> smem_set{0u};
-    return line_launch<RhsLineShape<DIM, NP>>(rhs_line_kernel<DIM, NP, NS, BLEND, BC>, smem_set, s, m, a, P, T);
+    return line_launch<RhsLineShape<DIM, NP>>(rhs_line_kernel<DIM, NP, NS, BLEND, BC, REF>, smem_set, s, m, a, P, T);
 }
 template <int NP, typename W>
 LineD<W> line_d(const OpTables &T) {
@@ -1148,10 +1252,10 @@ LineD<W> line_d(const OpTables &T) {
     for (int q = 0; q < NP * NP; ++q) D.d[q] = W(T.D[q]);
     return D;
 }
-template <int DIM, int NP, bool BC, typename W>
+template <int DIM, int NP, bool BC, typename W, bool REF = false>
 cudaError_t lift_line_launch(const MeshDev &m, const LiftArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {
     static std::atomic<unsigned> smem_set{0u};
-    return line_launch<LiftLineShape<DIM, NP, W>>(lift_line_kernel<DIM, NP, BC, W>, smem_set, s, m, a, P, line_d<NP, W>(T), T.w[0]);
+    return line_launch<LiftLineShape<DIM, NP, W>>(lift_line_kernel<DIM, NP, BC, REF, W>, smem_set, s, m, a, P, line_d<NP, W>(T), T.w[0]);
 }
 template <int DIM, int NP, bool NS>
 cudaError_t rhs_line_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T, cudaStream_t s) {

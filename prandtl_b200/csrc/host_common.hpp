@@ -325,7 +325,7 @@ inline prandtl_status check_viscous_bcs(const prandtl_mesh_desc *md, const prand
 // scaled normal must be the outward adjugate row of both its elements
 // (Nanson's formula for affine elements): nor = s1 adj(J_e1)[d1] =
 // -s2 adj(J_e2)[d2] with s = +1 on a local face 2d+1, -1 on 2d.
-inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::string &msg) {
+inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::string &msg, double tol = 1e-9) {
     const int dim = md->dim;
     for (int f = 0; f < md->num_faces; ++f) {
         const int *fe = md->face_elems + 4 * f;
@@ -340,7 +340,7 @@ inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::strin
                 err = std::fmax(err, std::fabs(nor[c] - sg * row[c]));
                 mag = std::fmax(mag, std::fabs(row[c]));
             }
-            if (!(err <= 1e-9 * mag)) {
+            if (!(err <= tol * mag)) {
                 msg = "face " + std::to_string(f) +
                       ": scaled normal differs from the element's adjugate row (non-affine or inconsistent mesh)";
                 return PRANDTL_EUNSUPPORTED;

@@ -60,6 +60,7 @@ struct prandtl_handle {
     unsigned long long *d_lambda = nullptr;
     unsigned int *d_health = nullptr;             // sticky state-check bits of the RK stages
     unsigned int *h_health = nullptr;             // pinned host copy of d_health
+    bool ref_lines = false;                       // MeshDev::ref_lines
     BcDev *d_bcs = nullptr;                       // boundary conditions
     // axisymmetric form: node coordinates [2][Ndof], axis-node flags, and the
     // state U recovered from the r-weighted RK state before each RHS
@@ -356,6 +357,7 @@ MeshDev mesh_dev(const prandtl_handle *h) {
     m.ngeo = h->d_ngeo;
     m.fnn = h->d_fnn;
     m.snor = h->d_snor;
+    m.ref_lines = h->ref_lines;
     return m;
 }
 
@@ -623,7 +625,14 @@ prandtl_status prandtl_create(const prandtl_mesh_desc *md, const prandtl_config 
     if ((st = dalloc(h, &h->d_out, S, "state out")) != PRANDTL_OK) return bail(st);
     if ((st = dalloc(h, &h->d_rk1, S, "rk register 1")) != PRANDTL_OK) return bail(st);
     if ((st = dalloc(h, &h->d_rk2, S, "rk register 2")) != PRANDTL_OK) return bail(st);
-    if (cfg->parabolic && cfg->precision == 0 && (st = dalloc(h, &h->d_grad, (size_t)dim * S, "gradients")) != PRANDTL_OK)
+    if (cfg->parabolic && cfg->precision == 0 && cfg->quirks == 0 && cfg->num_bcs == 0 && !cfg->blending && !mesh_curved(md)) {
+        std::string why;   // normals within rounding of the adjugate rows (which the lines use in their place)
+        h->ref_lines = check_face_normals(md, why, 1e-13) == PRANDTL_OK;
+    }
+    // reference mode by lines: viscous rows of every node, then of every face node
+    const size_t rows = (size_t)dim * (h->nf - 1) * h->Ndof;
+    const size_t ngrad = std::max((size_t)dim * S, h->ref_lines ? rows + 2 * rows / h->Np : 0);
+    if (cfg->parabolic && cfg->precision == 0 && (st = dalloc(h, &h->d_grad, ngrad, "gradients")) != PRANDTL_OK)
         return bail(st);
     if (cfg->parabolic && cfg->precision == 1 && (st = dalloc(h, &h->d_grad32, (size_t)dim * S, "gradients")) != PRANDTL_OK)
         return bail(st);

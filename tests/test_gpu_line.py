@@ -65,3 +65,21 @@ def test_boundaries(oracle_mod, dim, order, blending):
         d = op.Mult(u, np.empty_like(u))
         assert normalized_error(d, r["dudt"], mesh.num_fields) <= 1e-12
         op.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1.0 + 1e-6])
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_reference_mode_navier_stokes(oracle_mod, dim, order, scale):
+    """The reference's own viscous terms by lines, on each branch of the means;
+    with normals that are not the adjugate rows (scale) by the general form."""
+    from prandtl_b200.operator import DGSEMOperator
+    for k, (n, amp) in enumerate(zip(SHAPES[dim], (0.003, 0.1, 0.4))):
+        mesh = periodic_box(dim, n, order, 0.0, tuple(0.5 * c for c in n))
+        mesh.face_nor = mesh.face_nor * scale
+        u = state(mesh, amp, 20 * order + k)
+        r = oracle_mod.Oracle(mesh, quirks=0, parabolic=1, mu=0.01).rhs(u)
+        op = DGSEMOperator(mesh, quirks="reference", parabolic=True, mu=0.01)
+        d = op.Mult(u, np.empty_like(u))
+        assert normalized_error(d, r["dudt"], mesh.num_fields) <= 1e-12, (n, amp)
+        op.close()

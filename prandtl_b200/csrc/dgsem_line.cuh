@@ -137,6 +137,12 @@ __device__ __forceinline__ double ldg_now(const double *p) {
     return v;
 }
 
+// Brings the lines that hold p[0..n) into L2, spread over the NL lanes of an
+// element, without a register or a wait: for operands read later from DRAM.
+__device__ __forceinline__ void prefetch_l2(const double *p, int n, int ln, int nl) {
+    for (int q = 16 * ln; q < n; q += 16 * nl) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + q));
+}
+
 // Two-point flux along the metric row m (ChandrashekarFlux.cpp:11-83) of nodes
 // (rho, v, beta), rearranged: with q = (x+y)/(2 mean) of rho and beta and
 // rs = 1/(beta_a + beta_b), the enthalpy term p_hat/rho_ln + 1/(2(g-1) beta_ln)
@@ -403,6 +409,14 @@ __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysPara
             for (int f = 0; f < NF; ++f) s[i][f] = ldg_now(a.u + f * Ndof + e0 + ln + NL * i);
 #pragma unroll
         for (int k = 0; k < NG; ++k) g[k] = __ldg(a.geo + (long long)e * (DIM * DIM + 1) + min(ln + k * NL, DIM * DIM));
+        // what is read after the two-point fluxes: the element's viscous rows (32^3
+        // Np = 4: 157 -> 148 us) and, of states that leave L2 between stages (above
+        // 3 M values, 24 MB: the stage touches three to four times that), the stage
+        // update's other operand (256^2 step 160 -> 156 us; smaller states, 1 % slower)
+        if constexpr (NS) prefetch_l2(reinterpret_cast<const double *>(a.grad) + e0 * (DIM * (NF - 1)), DIM * (NF - 1) * ND, ln, NL);
+        if (NF * Ndof > 3000000 && (a.mode == EPI_LSRK ? a.rkA != 0.0 : a.mode >= EPI_SSP2))
+#pragma unroll
+            for (int f = 0; f < NF; ++f) prefetch_l2((a.mode == EPI_LSRK ? a.du : a.x0) + f * Ndof + e0, ND, ln, NL);
 #pragma unroll
         for (int k = 0; k < NB; ++k)
 #pragma unroll

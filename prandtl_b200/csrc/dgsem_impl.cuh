@@ -2,6 +2,11 @@
 // each dgsem_inst_*.cu translation unit instantiates one dimension, working
 // precision and physics).
 //
+// The FP64 RHS on affine meshes and the liftings with contravariant viscous
+// rows run by lines (dgsem_line.cuh).  The general form below runs the others:
+// the FP32-bulk RHS, non-affine and axisymmetric meshes, and Navier-Stokes with
+// gradients (the reference mode in batches, in FP32, with blending or boundaries).
+//
 // RHS: one lane group (a warp, or a power-of-two part of one for small
 // elements) per element.  Everything an element needs stays in shared memory
 // for the whole evaluation:

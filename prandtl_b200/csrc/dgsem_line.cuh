@@ -14,11 +14,11 @@
 // Here a node's primitives are read once per direction instead of once per
 // pair, no two-point or face flux goes through shared memory, every lane has
 // work in every phase and boundary and blending code is compiled in only where
-// it is used: half the warp instructions (157 M -> 79 M at 32^3 Np = 4).  What
-// bounds it now is FP64 issue (47 % of the pipe) and the latency of the global
+// it is used: half the warp instructions (157 M -> 73 M at 32^3 Np = 4).  What
+// bounds it now is FP64 issue (49 % of the pipe) and the latency of the global
 // loads at 12 warps per SM.  Measured, one launch:
-//   3D Np = 4 Navier-Stokes, 32^3 elements   324 -> 157 us
-//   3D Np = 5 Navier-Stokes, 15^3            103 ->  53 us
+//   3D Np = 4 Navier-Stokes, 32^3 elements   324 -> 147 us
+//   3D Np = 5 Navier-Stokes, 15^3            103 ->  49 us
 //   3D Np = 4 Euler, 24^3                    114 ->  52 us
 //   2D Np = 4 Euler, blended, 256^2          107 ->  57 us
 //   2D Np = 5 Euler, 101^2                    35 ->  23 us
@@ -374,7 +374,7 @@ __device__ __forceinline__ void line_boundary(const ElemIO &a, const PhysParams 
 // (DGSEMIntegrator.cpp:620), and the face nodes' own (lift_line_element).  The
 // general form reads 15 gradients per node, twice per face node, and evaluates
 // viscous fluxes from them at 12 warps per SM; here 18 values per node pass
-// through memory.  20^3 Np = 4: RHS 145 -> 66 us, lifting 49 -> 40 us.
+// through memory.  20^3 Np = 4: RHS 145 -> 57 us, lifting 49 -> 40 us.
 template <int DIM, int NP, bool NS, bool BLEND, bool BC, bool REF, typename Sync>
 __device__ __forceinline__ void rhs_line_element(const ElemIO &a, const PhysParams &P, const OpTables &T, int e, bool ok,
                                                  double *sH, int ln, const Sync &sync) {

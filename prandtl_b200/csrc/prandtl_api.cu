@@ -632,8 +632,16 @@ prandtl_status prandtl_create(const prandtl_mesh_desc *md, const prandtl_config 
     // reference mode by lines: viscous rows of every node, then of every face node
     const size_t rows = (size_t)dim * (h->nf - 1) * h->Ndof;
     const size_t ngrad = std::max((size_t)dim * S, h->ref_lines ? rows + 2 * rows / h->Np : 0);
-    if (cfg->parabolic && cfg->precision == 0 && (st = dalloc(h, &h->d_grad, ngrad, "gradients")) != PRANDTL_OK)
-        return bail(st);
+    if (cfg->parabolic && cfg->precision == 0) {
+        st = dalloc(h, &h->d_grad, ngrad, "gradients");
+        if (st == PRANDTL_ENOMEM && h->ref_lines) {   // no room for the face rows: the gradient form needs less
+            cudaGetLastError();
+            h->err.clear();
+            h->ref_lines = false;
+            st = dalloc(h, &h->d_grad, (size_t)dim * S, "gradients");
+        }
+        if (st != PRANDTL_OK) return bail(st);
+    }
     if (cfg->parabolic && cfg->precision == 1 && (st = dalloc(h, &h->d_grad32, (size_t)dim * S, "gradients")) != PRANDTL_OK)
         return bail(st);
     if ((st = dalloc(h, &h->d_alpha, (size_t)E, "alpha")) != PRANDTL_OK) return bail(st);

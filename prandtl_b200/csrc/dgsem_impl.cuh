@@ -1901,10 +1901,14 @@ __device__ __forceinline__ void lift_element(const ElemIO &a, const PhysParams &
 #pragma unroll
             for (int r = 0; r < DIM; ++r) Vc[r][f] += adj[r][cc] * val;
         });
+        // (affine elements: in line order, as rhs_element reads them)
 #pragma unroll
-        for (int r = 0; r < DIM; ++r)
+        for (int r = 0; r < DIM; ++r) {
+            const long long at = CURV ? r * (NF - 1) * Ndof + gnode
+                                      : ((long long)e * DIM + r) * ((NF - 1) * ND) + c[r] * (ND / NP) + line_index<DIM, NP>(r, c);
 #pragma unroll
-            for (int f = 1; f < NF; ++f) gout[(r * (NF - 1) + f - 1) * Ndof + gnode] = Vc[r][f];
+            for (int f = 1; f < NF; ++f) gout[at + (f - 1) * (CURV ? Ndof : (long long)ND)] = Vc[r][f];
+        }
     } else {
 #pragma unroll
         for (int q = 0; q < DIM; ++q)
@@ -2094,9 +2098,19 @@ cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &
     return cudaErrorInvalidValue;
 }
 // The FP64 forms on affine meshes run by lines (dgsem_line.cuh), but for
-// Navier-Stokes with gradients and the axisymmetric form.
+// Navier-Stokes with gradients, the axisymmetric form and small 2D meshes.
 template <bool NS, bool VC, typename Real>
 constexpr bool line_form() { return sizeof(Real) == 8 && (VC || !NS); }
+// Small 2D meshes stay with the general form in FP64: it gives an element's
+// nodes a lane each, the lines an element Np lanes, and below three warps of
+// lines per SM their longer serial chain counts.  SSP-RK3 step, general against
+// lines: vortex 32^2 N=3 22.5 / 25.8 us, N=4 24.9 / 39.1, 64^2 N=4 44.4 / 41.2,
+// 48^2 N=5 39.7 / 50.4, 64^2 N=5 63.7 / 53.1; at N=1 the lines are always ahead
+// (21.8 / 16.1).
+template <int DIM, int NP, typename Real>
+bool small_2d(const MeshDev &m) {
+    return DIM == 2 && NP > 2 && sizeof(Real) == 8 && (long long)m.E * NP < 15000;
+}
 // non-affine meshes (m.ngeo set) run the per-node-geometry kernels (FP64, or FP32-bulk Euler)
 template <int DIM, int NP, bool NS, bool VC, typename Real>
 cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
@@ -2109,9 +2123,9 @@ cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams 
         if (m.ref_lines && !P.blending) return rhs_line_launch<DIM, NP, true, false, false, true>(m, a, P, T, s);
     }
     if constexpr (line_form<NS, VC, Real>()) {   // by lines, but for the axisymmetric form
-        if (DIM == 3 || NS || !m.rad) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
+        if (DIM == 3 || (!m.rad && !small_2d<DIM, NP, Real>(m))) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
     }
-    if constexpr (sizeof(Real) == 4 || (NS && !VC) || (DIM == 2 && !NS))
+    if constexpr (sizeof(Real) == 4 || (NS && !VC) || DIM == 2)
         return P.blending || m.bcs ? rhs_launch_np<DIM, NP, NS, VC, Real, true, false>(m, a, P, T, s)
                                    : rhs_launch_np<DIM, NP, NS, VC, Real, false, false>(m, a, P, T, s);
     else return cudaErrorNotSupported;
@@ -2141,6 +2155,9 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
     }
     if constexpr (sizeof(Out) == 8 && !VC) {
         if (m.ref_lines && !P.blending) return lift_line_launch<DIM, NP, false, Out, true>(m, a, P, T, s);
+    }
+    if constexpr (VC && DIM == 2 && sizeof(Out) == 8) {
+        if (small_2d<DIM, NP, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
     }
     if constexpr (VC)
         return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)

@@ -83,3 +83,28 @@ def test_reference_mode_navier_stokes(oracle_mod, dim, order, scale):
         d = op.Mult(u, np.empty_like(u))
         assert normalized_error(d, r["dudt"], mesh.num_fields) <= 1e-12, (n, amp)
         op.close()
+
+
+# 2D meshes above the size from which lines run (15,000 lines per direction), odd
+LARGE_2D = {2: (101, 53), 3: (61, 67), 4: (59, 53), 5: (53, 49)}
+
+
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("order", [2, 3, 4, 5])
+def test_large_2d(oracle_mod, order, walls):
+    """2D by lines: partly filled last groups, each branch of the means, blending
+    and boundaries."""
+    from prandtl_b200.operator import DGSEMOperator
+    n = LARGE_2D[order]
+    kinds = [("slip_wall",), ("outflow",)] if walls else None
+    mesh = periodic_box(2, n, order, 0.0, tuple(0.5 * c for c in n), bcs=[0, 1, 1, 0] if walls else None)
+    for k, phys in enumerate((dict(), dict(blending=True), dict(parabolic=True, mu=0.01))):
+        u = state(mesh, (0.003, 0.4, 0.1)[k], 30 * order + k)
+        if walls and phys.get("parabolic"):
+            kinds = [("noslip_adiabatic", dict(wall_vel=(0.1, 0.0), heat_flux=0.02)), ("outflow",)]
+        r = oracle_mod.Oracle(mesh, quirks=1, bcs=kinds, **{a: (int(b) if isinstance(b, bool) else b)
+                                                            for a, b in phys.items()}).rhs(u)
+        op = DGSEMOperator(mesh, quirks="fixed", bcs=kinds, **phys)
+        d = op.Mult(u, np.empty_like(u))
+        assert normalized_error(d, r["dudt"], mesh.num_fields) <= 1e-12, phys
+        op.close()

@@ -114,9 +114,12 @@ __device__ __noinline__ double log_q_far(double x, double y, double f, double u)
     return 0.5 * log(y / x) / f;
 }
 
-// sqrt(x) for x >= 0: hardware estimate of 1/sqrt (PTX rsqrt.approx.ftz.f64)
-// refined by a coupled (Goldschmidt) iteration (Markstein, IBM J. Res. Dev. 34
-// (1990) 111-119), without special-value paths; 0 below 1e-300.
+// sqrt(x): hardware estimate of 1/sqrt (PTX rsqrt.approx.ftz.f64) refined by a
+// coupled (Goldschmidt) iteration (Markstein, IBM J. Res. Dev. 34 (1990)
+// 111-119).  Outside the positive normal numbers, which one integer compare of
+// the high word tells, as sqrt has it: NaN for negative arguments (a state
+// without a speed of sound must not look like one), zero, infinity and NaN
+// themselves; subnormals too come back as they are, within 2e-154 of their root.
 __device__ __forceinline__ double sqrt_pos(double x) {
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -126,7 +129,8 @@ __device__ __forceinline__ double sqrt_pos(double x) {
     h = fma(h, e, h);
     const double d = fma(-g, g, x);
     g = fma(d, h, g);
-    return x < 1e-300 ? 0.0 : g;
+    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) g = x < 0.0 ? nan("") : x;
+    return g;
 }
 
 // A load that stays where it is written: the compiler may not sink it to its
@@ -809,7 +813,7 @@ struct LineD {
     W d[36];
 };
 
-// ln(x / x0) for x, x0 > 0.
+// ln(x / x0) for x0 > 0; NaN for x < 0 (u > 1 there: the logarithm).
 __device__ __forceinline__ double log_ratio(double x, double x0) {
     const double f = (x - x0) * rcp(x + x0), u = f * f;
     double q = 1.0 / 11.0;
@@ -834,6 +838,9 @@ __device__ __forceinline__ LineRef line_ref(const double *s, const PhysParams &P
     R.p = P.gammaM1 * fma(-0.5 * mm, r, s[1 + DIM]);
     R.beta = s[0] * rcp(R.p);
     R.bvsq = R.beta * (0.5 * mm * r * r);
+    // a reference node without entropy variables leaves the others theirs, and
+    // log_ratio needs a positive one: absolute values then
+    if (!(s[0] > 0.0 && R.beta > 0.0 && R.beta < 1e300)) R = LineRef{1.0, 1.0, 0.0, 0.0};
     return R;
 }
 template <int DIM>

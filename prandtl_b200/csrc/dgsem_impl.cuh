@@ -2156,8 +2156,11 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
     if constexpr (sizeof(Out) == 8 && !VC) {
         if (m.ref_lines && !P.blending) return lift_line_launch<DIM, NP, false, Out, true>(m, a, P, T, s);
     }
-    if constexpr (VC && DIM == 2 && sizeof(Out) == 8) {
-        if (small_2d<DIM, NP, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
+    // the lines take the adjugate rows for the normals: in FP64 only where they are
+    // the same within rounding (FP32's own rounding, 6e-8, covers the 1e-9 that
+    // meshes may be off by)
+    if constexpr (VC && sizeof(Out) == 8) {
+        if (!m.nor_rows || small_2d<DIM, NP, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
     }
     if constexpr (VC)
         return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)
@@ -2204,41 +2207,56 @@ cudaError_t rhs_batch_launch_np(int grid, const BatchClassDev &c, const BatchSta
         return cudaGetLastError();
     }
 }
-template <int DIM, int NP, typename Out, bool VC, bool FEAT>
-cudaError_t lift_batch_prepare_np(BatchKernelInfo *info) {
+// Liftings with contravariant viscous rows by lines; in FP64 on meshes whose
+// normals are not the adjugate rows within rounding, and with gradients, node by node.
+template <int DIM, int NP, typename Out, bool VC>
+cudaError_t lift_batch_prepare_np(bool feat, bool nor_rows, BatchKernelInfo *info) {
     if constexpr (VC) {
         using L = LiftLineShape<DIM, NP, Out>;
-        return line_batch_prepare<L>((const void *)lift_line_batch_kernel<DIM, NP, FEAT, Out>, line_batch_smem<L>(), info);
-    } else {
-    using S = LiftBatchShape<DIM, NP, Out>;
-    const size_t sm = lift_batch_smem<DIM, NP, Out>();
-    cudaError_t err = cudaFuncSetAttribute(lift_batch_kernel<DIM, NP, Out, VC>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (err != cudaSuccess) return err;
-    int nb = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, lift_batch_kernel<DIM, NP, Out, VC>, S::THREADS, sm);
-    if (err != cudaSuccess) return err;
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, lift_batch_kernel<DIM, NP, Out, VC>);
-    info->blocks_per_sm = nb;
-    info->threads = S::THREADS;
-    info->smem = (int)sm;
-    info->regs = fa.numRegs;
-    info->elems_per_item = S::EPB;
-    return cudaSuccess;
+        if (sizeof(Out) == 4 || nor_rows)
+            return line_batch_prepare<L>(feat ? (const void *)lift_line_batch_kernel<DIM, NP, true, Out>
+                                              : (const void *)lift_line_batch_kernel<DIM, NP, false, Out>,
+                                         line_batch_smem<L>(), info);
     }
+    if constexpr (!VC || sizeof(Out) == 8) {
+        using S = LiftBatchShape<DIM, NP, Out>;
+        const size_t sm = lift_batch_smem<DIM, NP, Out>();
+        cudaError_t err = cudaFuncSetAttribute(lift_batch_kernel<DIM, NP, Out, VC>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (err != cudaSuccess) return err;
+        int nb = 0;
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, lift_batch_kernel<DIM, NP, Out, VC>, S::THREADS, sm);
+        if (err != cudaSuccess) return err;
+        cudaFuncAttributes fa{};
+        cudaFuncGetAttributes(&fa, lift_batch_kernel<DIM, NP, Out, VC>);
+        info->blocks_per_sm = nb;
+        info->threads = S::THREADS;
+        info->smem = (int)sm;
+        info->regs = fa.numRegs;
+        info->elems_per_item = S::EPB;
+        return cudaSuccess;
+    }
+    return cudaErrorNotSupported;
 }
-template <int DIM, int NP, typename Out, bool VC, bool FEAT>
-cudaError_t lift_batch_launch_np(int grid, const BatchClassDev &c, const BatchStage &st, const OpTables &T,
-                                 cudaStream_t s) {
+template <int DIM, int NP, typename Out, bool VC>
+cudaError_t lift_batch_launch_np(bool feat, bool nor_rows, int grid, const BatchClassDev &c, const BatchStage &st,
+                                 const OpTables &T, cudaStream_t s) {
     if constexpr (VC) {
         using L = LiftLineShape<DIM, NP, Out>;
-        lift_line_batch_kernel<DIM, NP, FEAT, Out><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, line_d<NP, Out>(T), T.w[0]);
-    } else {
+        if (sizeof(Out) == 4 || nor_rows) {
+            if (feat)
+                lift_line_batch_kernel<DIM, NP, true, Out><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, line_d<NP, Out>(T), T.w[0]);
+            else
+                lift_line_batch_kernel<DIM, NP, false, Out><<<grid, L::THREADS, line_batch_smem<L>(), s>>>(c, st, line_d<NP, Out>(T), T.w[0]);
+            return cudaGetLastError();
+        }
+    }
+    if constexpr (!VC || sizeof(Out) == 8) {
         using S = LiftBatchShape<DIM, NP, Out>;
         lift_batch_kernel<DIM, NP, Out, VC><<<grid, S::THREADS, lift_batch_smem<DIM, NP, Out>(), s>>>(c, st, T);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    return cudaErrorNotSupported;
 }
 
 }   // namespace
@@ -2286,15 +2304,13 @@ cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const 
     }()))
 }
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_prepare(int order, bool feat, BatchKernelInfo *info) {
-    PRANDTL_ORDER_SWITCH((feat ? lift_batch_prepare_np<DIM, NP, Out, VC, true>(info)
-                               : lift_batch_prepare_np<DIM, NP, Out, VC, false>(info)))
+cudaError_t lift_batch_prepare(int order, bool feat, bool nor_rows, BatchKernelInfo *info) {
+    PRANDTL_ORDER_SWITCH((lift_batch_prepare_np<DIM, NP, Out, VC>(feat, nor_rows, info)))
 }
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_launch(int order, bool feat, int grid, const BatchClassDev &c, const BatchStage &st,
+cudaError_t lift_batch_launch(int order, bool feat, bool nor_rows, int grid, const BatchClassDev &c, const BatchStage &st,
                               const OpTables &T, cudaStream_t s) {
-    PRANDTL_ORDER_SWITCH((feat ? lift_batch_launch_np<DIM, NP, Out, VC, true>(grid, c, st, T, s)
-                               : lift_batch_launch_np<DIM, NP, Out, VC, false>(grid, c, st, T, s)))
+    PRANDTL_ORDER_SWITCH((lift_batch_launch_np<DIM, NP, Out, VC>(feat, nor_rows, grid, c, st, T, s)))
 }
 
 // One translation unit per (DIM, Real, physics) instantiates its share.
@@ -2307,8 +2323,8 @@ cudaError_t lift_batch_launch(int order, bool feat, int grid, const BatchClassDe
 #define PRANDTL_INSTANTIATE_LIFT(DIMV, OUT, VCV)                                                        \
     template cudaError_t lift_dispatch<DIMV, OUT, VCV>(int, const MeshDev &, const LiftArgs &,          \
                                                        const PhysParams &, const OpTables &, cudaStream_t); \
-    template cudaError_t lift_batch_prepare<DIMV, OUT, VCV>(int, bool, BatchKernelInfo *);                    \
-    template cudaError_t lift_batch_launch<DIMV, OUT, VCV>(int, bool, int, const BatchClassDev &, const BatchStage &, \
+    template cudaError_t lift_batch_prepare<DIMV, OUT, VCV>(int, bool, bool, BatchKernelInfo *);              \
+    template cudaError_t lift_batch_launch<DIMV, OUT, VCV>(int, bool, bool, int, const BatchClassDev &, const BatchStage &, \
                                                            const OpTables &, cudaStream_t);
 
 }   // namespace prandtl

@@ -64,19 +64,19 @@ cudaError_t batch_prepare_rhs(int dim, int order, bool ns, bool vc, bool fp32, i
     if (fp32) PRANDTL_DIM_PHYS(rhs_batch_prepare, float, ns, vc, order, variant, feat, info);
     PRANDTL_DIM_PHYS(rhs_batch_prepare, double, ns, vc, order, variant, feat, info);
 }
-cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, bool feat, BatchKernelInfo *info) {
-    if (fp32) PRANDTL_DIM_LIFT(lift_batch_prepare, float, vc, order, feat, info);
-    PRANDTL_DIM_LIFT(lift_batch_prepare, double, vc, order, feat, info);
+cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, bool feat, bool nor_rows, BatchKernelInfo *info) {
+    if (fp32) PRANDTL_DIM_LIFT(lift_batch_prepare, float, vc, order, feat, nor_rows, info);
+    PRANDTL_DIM_LIFT(lift_batch_prepare, double, vc, order, feat, nor_rows, info);
 }
 cudaError_t batch_launch_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat, int grid,
                              const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s) {
     if (fp32) PRANDTL_DIM_PHYS(rhs_batch_launch, float, ns, vc, order, variant, feat, grid, c, st, T, s);
     PRANDTL_DIM_PHYS(rhs_batch_launch, double, ns, vc, order, variant, feat, grid, c, st, T, s);
 }
-cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, bool feat, int grid, const BatchClassDev &c,
-                              const BatchStage &st, const OpTables &T, cudaStream_t s) {
-    if (fp32) PRANDTL_DIM_LIFT(lift_batch_launch, float, vc, order, feat, grid, c, st, T, s);
-    PRANDTL_DIM_LIFT(lift_batch_launch, double, vc, order, feat, grid, c, st, T, s);
+cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, bool feat, bool nor_rows, int grid,
+                              const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s) {
+    if (fp32) PRANDTL_DIM_LIFT(lift_batch_launch, float, vc, order, feat, nor_rows, grid, c, st, T, s);
+    PRANDTL_DIM_LIFT(lift_batch_launch, double, vc, order, feat, nor_rows, grid, c, st, T, s);
 }
 
 namespace {

@@ -16,6 +16,11 @@ enum EpilogueMode : int {
     EPI_SSP3 = 4,    // u_out = 1/3 x0 + 2/3 (u + dt L(u))       (stage 3; u_out may be x0)
 };
 
+// Largest difference between a face's scaled normal and its elements' adjugate
+// rows, of the row's largest entry: what the Navier-Stokes form with
+// contravariant viscous fluxes admits, and what counts as rounding.
+constexpr double NORMAL_TOL = 1e-9, NORMAL_ROWS_TOL = 1e-13;
+
 struct MeshDev {
     const double *geo;   // [E][DIM*DIM + 1]: adj(J) row-major, then det J
     const int4 *nbr;     // [E][2*DIM]: {neighbour elem, neighbour local face, face id, role}
@@ -34,9 +39,12 @@ struct MeshDev {
     const double *ngeo;
     const double *fnn;
     const double *snor;
+    // affine meshes: the scaled normals are the elements' adjugate rows within
+    // rounding (NORMAL_ROWS_TOL), which the FP64 lifting by lines takes in their place
+    bool nor_rows = false;
     // FP64 Navier-Stokes in the reference mode: run by lines.  The mesh has no
-    // boundary conditions, its normals are the elements' adjugate rows, and the
-    // gradient buffer holds DIM (NF-1) (1 + 2/Np) values per node
+    // boundary conditions, nor_rows holds, and the gradient buffer has
+    // DIM (NF-1) (1 + 2/Np) values per node
     bool ref_lines = false;
 };
 
@@ -126,14 +134,16 @@ bool order_supported(int dim, int order);
 // RHS launch shape.  `vc` selects the Navier-Stokes form that passes
 // contravariant viscous fluxes from the lifting to the RHS (quirks = 1) instead
 // of primitive gradients (quirks = 0).  `feat`: the class's solves have blending
-// or boundary conditions (their code is compiled out of the other kernels).  prepare_* must run outside stream capture.
+// or boundary conditions (their code is compiled out of the other kernels).
+// `nor_rows` as in MeshDev, for the class's meshes (FP64 liftings).  prepare_*
+// must run outside stream capture.
 int batch_num_variants();
 cudaError_t batch_prepare_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat,
                               BatchKernelInfo *info);
-cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, bool feat, BatchKernelInfo *info);
+cudaError_t batch_prepare_lift(int dim, int order, bool vc, bool fp32, bool feat, bool nor_rows, BatchKernelInfo *info);
 cudaError_t batch_launch_rhs(int dim, int order, bool ns, bool vc, bool fp32, int variant, bool feat, int grid,
                              const BatchClassDev &c, const BatchStage &st, const OpTables &T, cudaStream_t s);
-cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, bool feat, int grid, const BatchClassDev &c,
+cudaError_t batch_launch_lift(int dim, int order, bool vc, bool fp32, bool feat, bool nor_rows, int grid, const BatchClassDev &c,
                               const BatchStage &st, const OpTables &T, cudaStream_t s);
 // End of a batch step: every live solve with steps left advances its counters,
 // flips its LSRK parity, (cfl > 0) takes its next dt from lambda, and writes
@@ -175,9 +185,9 @@ template <int DIM, typename Real, bool NS, bool VC>
 cudaError_t rhs_batch_launch(int order, int variant, bool feat, int grid, const BatchClassDev &c,
                              const BatchStage &st, const OpTables &T, cudaStream_t s);
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_prepare(int order, bool feat, BatchKernelInfo *info);
+cudaError_t lift_batch_prepare(int order, bool feat, bool nor_rows, BatchKernelInfo *info);
 template <int DIM, typename Out, bool VC>
-cudaError_t lift_batch_launch(int order, bool feat, int grid, const BatchClassDev &c, const BatchStage &st,
+cudaError_t lift_batch_launch(int order, bool feat, bool nor_rows, int grid, const BatchClassDev &c, const BatchStage &st,
                               const OpTables &T, cudaStream_t s);
 
 // The Navier-Stokes form used for a configuration: contravariant viscous

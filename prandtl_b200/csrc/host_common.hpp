@@ -324,9 +324,12 @@ inline prandtl_status check_viscous_bcs(const prandtl_mesh_desc *md, const prand
 // For the Navier-Stokes form with contravariant viscous fluxes: every face's
 // scaled normal must be the outward adjugate row of both its elements
 // (Nanson's formula for affine elements): nor = s1 adj(J_e1)[d1] =
-// -s2 adj(J_e2)[d2] with s = +1 on a local face 2d+1, -1 on 2d.
-inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::string &msg, double tol = 1e-9) {
+// -s2 adj(J_e2)[d2] with s = +1 on a local face 2d+1, -1 on 2d.  Meshes are
+// taken up to NORMAL_TOL; `rows` tells whether the normals are the rows within
+// rounding (NORMAL_ROWS_TOL), so that FP64 kernels may put the rows in their place.
+inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::string &msg, bool &rows) {
     const int dim = md->dim;
+    rows = true;
     for (int f = 0; f < md->num_faces; ++f) {
         const int *fe = md->face_elems + 4 * f;
         const double *nor = md->face_nor + (size_t)f * dim;
@@ -340,7 +343,9 @@ inline prandtl_status check_face_normals(const prandtl_mesh_desc *md, std::strin
                 err = std::fmax(err, std::fabs(nor[c] - sg * row[c]));
                 mag = std::fmax(mag, std::fabs(row[c]));
             }
-            if (!(err <= tol * mag)) {
+            if (err > NORMAL_ROWS_TOL * mag) rows = false;
+            if (!(err <= NORMAL_TOL * mag)) {
+                rows = false;
                 msg = "face " + std::to_string(f) +
                       ": scaled normal differs from the element's adjugate row (non-affine or inconsistent mesh)";
                 return PRANDTL_EUNSUPPORTED;
@@ -475,7 +480,7 @@ inline prandtl_status check_face_node_normals(const prandtl_mesh_desc *md, std::
                     err = std::fmax(err, std::fabs(nor[c] - sg * row[c]));
                     mag = std::fmax(mag, std::fabs(row[c]));
                 }
-                if (!(err <= 1e-9 * mag)) {
+                if (!(err <= NORMAL_TOL * mag)) {
                     msg = "face " + std::to_string(f) + " node " + std::to_string(a) +
                           ": scaled normal differs from the element's adjugate row there";
                     return PRANDTL_EUNSUPPORTED;

@@ -60,7 +60,7 @@ struct prandtl_handle {
     unsigned long long *d_lambda = nullptr;
     unsigned int *d_health = nullptr;             // sticky state-check bits of the RK stages
     unsigned int *h_health = nullptr;             // pinned host copy of d_health
-    bool ref_lines = false;                       // MeshDev::ref_lines
+    bool nor_rows = false, ref_lines = false;     // as in MeshDev
     BcDev *d_bcs = nullptr;                       // boundary conditions
     // axisymmetric form: node coordinates [2][Ndof], axis-node flags, and the
     // state U recovered from the r-weighted RK state before each RHS
@@ -357,6 +357,7 @@ MeshDev mesh_dev(const prandtl_handle *h) {
     m.ngeo = h->d_ngeo;
     m.fnn = h->d_fnn;
     m.snor = h->d_snor;
+    m.nor_rows = h->nor_rows;
     m.ref_lines = h->ref_lines;
     return m;
 }
@@ -564,6 +565,10 @@ prandtl_status prandtl_create(const prandtl_mesh_desc *md, const prandtl_config 
 
     const int dim = md->dim, E = md->num_elements, F = md->num_faces;
     std::vector<int4> nbr;
+    // reference mode by lines: without blending, boundary conditions and per-node geometry
+    const bool ref_plain = cfg->parabolic && cfg->precision == 0 && cfg->quirks == 0 && cfg->num_bcs == 0 &&
+                           !cfg->blending && !mesh_curved(md);
+    bool nor_rows = false;
     {
         std::string msg;
         prandtl_status vst = check_bcs(cfg, md->dim, msg);
@@ -575,7 +580,7 @@ prandtl_status prandtl_create(const prandtl_mesh_desc *md, const prandtl_config 
             vst = PRANDTL_EUNSUPPORTED;
         }
         if (vst == PRANDTL_OK && cfg->parabolic && cfg->quirks != 0)
-            vst = mesh_curved(md) ? check_face_node_normals(md, msg) : check_face_normals(md, msg);
+            vst = mesh_curved(md) ? check_face_node_normals(md, msg) : check_face_normals(md, msg, nor_rows);
         if (vst != PRANDTL_OK) return fail(nullptr, vst, msg);
     }
 
@@ -625,10 +630,12 @@ prandtl_status prandtl_create(const prandtl_mesh_desc *md, const prandtl_config 
     if ((st = dalloc(h, &h->d_out, S, "state out")) != PRANDTL_OK) return bail(st);
     if ((st = dalloc(h, &h->d_rk1, S, "rk register 1")) != PRANDTL_OK) return bail(st);
     if ((st = dalloc(h, &h->d_rk2, S, "rk register 2")) != PRANDTL_OK) return bail(st);
-    if (cfg->parabolic && cfg->precision == 0 && cfg->quirks == 0 && cfg->num_bcs == 0 && !cfg->blending && !mesh_curved(md)) {
-        std::string why;   // normals within rounding of the adjugate rows (which the lines use in their place)
-        h->ref_lines = check_face_normals(md, why, 1e-13) == PRANDTL_OK;
+    if (ref_plain) {
+        std::string why;   // other normals are no error here
+        check_face_normals(md, why, nor_rows);
     }
+    h->nor_rows = nor_rows;
+    h->ref_lines = ref_plain && nor_rows;
     // reference mode by lines: viscous rows of every node, then of every face node
     const size_t rows = (size_t)dim * (h->nf - 1) * h->Ndof;
     const size_t ngrad = std::max((size_t)dim * S, h->ref_lines ? rows + 2 * rows / h->Np : 0);

@@ -117,10 +117,12 @@ Layout solve_layout(int dim, int order, int E, int F, bool ns, bool blending, bo
     return L;
 }
 
-// feat: blending or boundary conditions, whose kernels differ; a class of its
-// own, so that a solve runs the same kernel whatever else the batch holds
-int class_key(int dim, int order, bool ns, bool vc, bool feat) {
-    return (((dim * 16 + order) * 2 + (ns ? 1 : 0)) * 2 + (vc ? 1 : 0)) * 2 + (feat ? 1 : 0);
+// feat: blending or boundary conditions, off_rows: FP64 liftings of meshes whose
+// normals are not their adjugate rows within rounding.  Their kernels differ: a
+// class of its own, so that a solve runs the same kernel whatever else the
+// batch holds
+int class_key(int dim, int order, bool ns, bool vc, bool feat, bool off_rows) {
+    return ((((dim * 16 + order) * 2 + (off_rows ? 1 : 0)) * 2 + (ns ? 1 : 0)) * 2 + (vc ? 1 : 0)) * 2 + (feat ? 1 : 0);
 }
 
 struct Solve {
@@ -139,6 +141,7 @@ struct Class {
     int dim = 0, order = 0;
     bool ns = false, vc = false;   // vc: NS with contravariant viscous fluxes (quirks = 1)
     bool feat = false;             // blending or boundary conditions
+    bool off_rows = false;         // normals off the adjugate rows: FP64 lifting along the normals
     OpTables T{};
     std::vector<int> ids;        // slot -> solve id
     int *d_buf = nullptr;        // ids[cap] | prefix[cap + 1] | hdr[4]
@@ -357,8 +360,8 @@ prandtl_status up_copy(prandtl_batch *b, void *dst, const void *src, size_t n) {
     return PRANDTL_OK;
 }
 
-prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc, bool feat, Class **out) {
-    const int key = class_key(dim, order, ns, vc, feat);
+prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc, bool feat, bool off_rows, Class **out) {
+    const int key = class_key(dim, order, ns, vc, feat, off_rows);
     auto it = b->classes.find(key);
     if (it != b->classes.end()) { *out = &it->second; return PRANDTL_OK; }
     Class c;
@@ -367,6 +370,7 @@ prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc,
     c.ns = ns;
     c.vc = vc;
     c.feat = feat;
+    c.off_rows = off_rows;
     build_tables(order, c.T);
     const bool fp32 = b->cfg.precision == 1;
     int first_ok = -1;
@@ -378,7 +382,7 @@ prandtl_status get_class(prandtl_batch *b, int dim, int order, bool ns, bool vc,
     if (first_ok < 0) return bfail(b, PRANDTL_EUNSUPPORTED, "no RHS launch shape fits this device");
     c.variant = first_ok;
     if (ns) {
-        BCK(b, batch_prepare_lift(dim, order, vc, fp32, feat, &c.linfo), "prepare batch lift kernel");
+        BCK(b, batch_prepare_lift(dim, order, vc, fp32, feat, !off_rows, &c.linfo), "prepare batch lift kernel");
         if (c.linfo.blocks_per_sm <= 0) return bfail(b, PRANDTL_EUNSUPPORTED, "lift kernel does not fit this device");
     }
     const size_t words = 2 * (size_t)b->cap + 5;
@@ -405,7 +409,7 @@ prandtl_status enqueue_step(prandtl_batch *b, cudaStream_t s) {
             Class &c = kv.second;
             if (c.ns) {
                 const int grid = c.linfo.blocks_per_sm * b->num_sms;
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, grid, c.dev, st, c.T, s), "batch lift launch");
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, !c.off_rows, grid, c.dev, st, c.T, s), "batch lift launch");
             }
             const int grid = c.rinfo[c.variant].blocks_per_sm * b->num_sms;
             BCK(b, batch_launch_rhs(c.dim, c.order, c.ns, c.vc, fp32, c.variant, c.feat, grid, c.dev, st, c.T, s),
@@ -441,7 +445,7 @@ prandtl_status tune_step(prandtl_batch *b, int v) {
             if (c.ns) {
                 const int grid = c.linfo.blocks_per_sm * b->num_sms;
                 BCK(b, cudaEventRecord(b->tev[q], b->stream), "event");
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, grid, c.dev, st, c.T, b->stream),
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, !c.off_rows, grid, c.dev, st, c.T, b->stream),
                     "batch lift launch");
                 BCK(b, cudaEventRecord(b->tev[q + 1], b->stream), "event");
             }
@@ -698,6 +702,7 @@ struct Prep {
     std::string msg;
     std::vector<int4> nbr;
     std::vector<double> geo;
+    bool nor_rows = true;   // the normals are the adjugate rows within rounding (viscous solves)
     // tables of a very large mesh are not kept for the next admission
     void trim() {
         if (nbr.capacity() * sizeof(int4) + geo.capacity() * sizeof(double) > (size_t(64) << 20)) {
@@ -733,7 +738,7 @@ void prep_solve(const prandtl_mesh_desc *md, const prandtl_config *cfg, const pr
         st = PRANDTL_EUNSUPPORTED;
         p.msg = "non-affine elements run on a prandtl_create FP64 operator, not in a batch";
     }
-    if (st == PRANDTL_OK && cfg->parabolic && cfg->quirks != 0) st = check_face_normals(md, p.msg);
+    if (st == PRANDTL_OK && cfg->parabolic && cfg->quirks != 0) st = check_face_normals(md, p.msg, p.nor_rows);
     if (st == PRANDTL_OK) geometry_rows_into(md, p.geo);
     p.st = st;
 }
@@ -747,11 +752,11 @@ prandtl_status admit_prepared(prandtl_batch *b, const prandtl_mesh_desc *md, con
     BCK(b, cudaSetDevice(b->device), "cudaSetDevice");
     const int dim = md->dim, order = md->order, E = md->num_elements, F = md->num_faces;
     const bool ns = cfg->parabolic != 0, fp32 = b->cfg.precision == 1, blend = cfg->blending != 0;
-    const bool vc = ns && cfg->quirks != 0, feat = blend || cfg->num_bcs > 0;
+    const bool vc = ns && cfg->quirks != 0, feat = blend || cfg->num_bcs > 0, off_rows = vc && !fp32 && !p.nor_rows;
     const Layout L = solve_layout(dim, order, E, F, ns, blend, fp32, cfg->num_bcs);
     if (b->free_ids.empty()) return bfail(b, PRANDTL_ENOMEM, "solve table full");
     Class *c = nullptr;
-    if ((st = get_class(b, dim, order, ns, vc, feat, &c)) != PRANDTL_OK) return st;
+    if ((st = get_class(b, dim, order, ns, vc, feat, off_rows, &c)) != PRANDTL_OK) return st;
     size_t off = 0;
     if (!b->alloc.alloc(L.total, &off))
         return bfail(b, PRANDTL_ENOMEM, "arena has no room: need " + std::to_string(L.total) +
@@ -763,7 +768,7 @@ prandtl_status admit_prepared(prandtl_batch *b, const prandtl_mesh_desc *md, con
     s.dim = dim;
     s.order = order;
     s.ns = ns;
-    s.key = class_key(dim, order, ns, vc, feat);
+    s.key = class_key(dim, order, ns, vc, feat, off_rows);
     s.E = E;
     s.nf = dim + 2;
     s.gamma = cfg->gamma;
@@ -1153,10 +1158,10 @@ prandtl_status prandtl_batch_tune(prandtl_batch *b, int reps) {
         if (c.ids.empty()) continue;
         if (c.ns) {
             const int lgrid = c.linfo.blocks_per_sm * b->num_sms;
-            BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
+            BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, !c.off_rows, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
             BCK(b, cudaEventRecord(b->ev0, b->stream), "event");
             for (int r = 0; r < reps; ++r)
-                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
+                BCK(b, batch_launch_lift(c.dim, c.order, c.vc, fp32, c.feat, !c.off_rows, lgrid, c.dev, st0, c.T, b->stream), "tune lift");
             BCK(b, cudaEventRecord(b->ev1, b->stream), "event");
             if ((st = bwait(b)) != PRANDTL_OK) return st;
             float lms = 0.f;
@@ -1193,8 +1198,8 @@ prandtl_status prandtl_batch_class_info(prandtl_batch *b, int dim, int order, in
     if (!b) return PRANDTL_EINVAL;
     std::lock_guard<std::mutex> lk(b->mu);
     auto it = b->classes.end();
-    for (int q = 0; q < 4 && it == b->classes.end(); ++q)   // plain solves first, vc before gradients
-        it = b->classes.find(class_key(dim, order, parabolic != 0, parabolic != 0 && !(q & 1), (q & 2) != 0));
+    for (int q = 0; q < 8 && it == b->classes.end(); ++q)   // plain solves first, vc before gradients
+        it = b->classes.find(class_key(dim, order, parabolic != 0, parabolic != 0 && !(q & 1), (q & 2) != 0, (q & 4) != 0));
     if (it == b->classes.end()) return bfail(b, PRANDTL_EINVAL, "no such class in this batch");
     if (variant) *variant = it->second.variant;
     if (n_variants) *n_variants = b->nvar;

@@ -97,8 +97,11 @@ __global__ void noalloc_geometry(const double *__restrict__ adj, const double *_
 }
 
 // Scatter every face into its two element slots; count faces that are out of
-// range, not aligned opposite faces, or land on an already-filled slot.
-__global__ void noalloc_faces(const int *__restrict__ faces, int F, int E, int dim,
+// range, not aligned opposite faces, or land on an already-filled slot (bad[0]),
+// and those whose scaled normal is not the adjugate row of both elements within
+// rounding (bad[1]; check_face_normals on the host).
+__global__ void noalloc_faces(const int *__restrict__ faces, const double *__restrict__ nor,
+                              const double *__restrict__ adj, int F, int E, int dim,
                               int4 *__restrict__ nbr, unsigned int *__restrict__ bad) {
     const int NFACE = 2 * dim;
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < F;
@@ -116,6 +119,19 @@ __global__ void noalloc_faces(const int *__restrict__ faces, int F, int E, int d
         if (atomicCAS(s2, -1, e1) != -1) { atomicAdd(bad, 1u); continue; }
         s1[1] = l2; s1[2] = (int)f; s1[3] = 0;
         s2[1] = l1; s2[2] = (int)f; s2[3] = 1;
+        bool rows = true;
+        for (int side = 0; side < 2; ++side) {
+            const int l = side ? l2 : l1;
+            const double sg = (l & 1) == side ? -1.0 : 1.0;
+            const double *row = adj + ((long long)(side ? e2 : e1) * dim + (l >> 1)) * dim;
+            double err = 0.0, mag = 0.0;
+            for (int c = 0; c < dim; ++c) {
+                err = fmax(err, fabs(nor[f * dim + c] - sg * row[c]));
+                mag = fmax(mag, fabs(row[c]));
+            }
+            rows = rows && err <= NORMAL_ROWS_TOL * mag;
+        }
+        if (!rows) atomicAdd(bad + 1, 1u);
     }
 }
 
@@ -179,7 +195,7 @@ extern "C" prandtl_status prandtl_rhs_noalloc(const prandtl_mesh_desc *m, const 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
     cudaError_t e;
-    if ((e = cudaMemsetAsync(bad, 0, sizeof(unsigned int), s)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned int), s)) != cudaSuccess)
         return fail(PRANDTL_ECUDA, cudaGetErrorString(e));
     const int tpb = 256;
     const int gE = (int)std::min<long long>((E + tpb - 1) / tpb, 4096);
@@ -187,18 +203,18 @@ extern "C" prandtl_status prandtl_rhs_noalloc(const prandtl_mesh_desc *m, const 
     const long long nslots = (long long)E * NFACE;
     const int gS = (int)std::min<long long>((nslots + tpb - 1) / tpb, 4096);
     noalloc_geometry<<<gE, tpb, 0, s>>>(m->elem_adj, m->elem_detj, geo, nbr, E, dim, bad);
-    noalloc_faces<<<gF, tpb, 0, s>>>(m->face_elems, F, E, dim, nbr, bad);
+    noalloc_faces<<<gF, tpb, 0, s>>>(m->face_elems, m->face_nor, m->elem_adj, F, E, dim, nbr, bad);
     noalloc_check<<<gS, tpb, 0, s>>>(nbr, nslots, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(PRANDTL_ECUDA, cudaGetErrorString(e));
-    // wait (bounded) for the check, then read its 4-byte count (a copy to
+    // wait (bounded) for the check, then read its two counts (a copy to
     // pageable memory returns once it has completed)
     if ((e = cudaEventRecord(check_done, s)) != cudaSuccess) return fail(PRANDTL_ECUDA, cudaGetErrorString(e));
     st = wait_event(check_done, cfg->timeout_s > 0 ? cfg->timeout_s : 120.0);
     if (st != PRANDTL_OK) return st;
-    unsigned int nbad = 0;
-    if ((e = cudaMemcpyAsync(&nbad, bad, sizeof(nbad), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+    unsigned int nbad[2] = {0, 0};
+    if ((e = cudaMemcpyAsync(nbad, bad, sizeof(nbad), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return fail(PRANDTL_ECUDA, cudaGetErrorString(e));
-    if (nbad != 0)
+    if (nbad[0] != 0)
         return fail(PRANDTL_EUNSUPPORTED,
                     "mesh invalid: faces out of range, duplicated or missing (only periodic meshes with aligned "
                     "faces), or a non-positive det J");
@@ -214,6 +230,7 @@ extern "C" prandtl_status prandtl_rhs_noalloc(const prandtl_mesh_desc *m, const 
     md.fnor = m->face_nor;
     md.E = E;
     md.Ndof = Ndof;
+    md.nor_rows = nbad[1] == 0;
     md.bcs = nullptr;   // periodic meshes only: boundary faces fail the check above
     if (cfg->parabolic) {
         LiftArgs la{u, grad};

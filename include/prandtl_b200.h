@@ -445,7 +445,9 @@ prandtl_status prandtl_batch_tune(prandtl_batch *b, int reps);
 prandtl_status prandtl_batch_tune_in_steps(prandtl_batch *b);
 /* Launch shape chosen for a class and the tuned times (ms per launch, -1 when
  * not timed) of each of the *n_variants RHS shapes and of the lifting launch;
- * ms and lift_ms may be NULL. */
+ * ms and lift_ms may be NULL.  Solves with and without blending or boundary
+ * conditions (and, in FP64, with normals off the adjugate rows) launch on
+ * their own: the times are their sums, the shape is that of the most elements. */
 prandtl_status prandtl_batch_class_info(prandtl_batch *b, int dim, int order, int parabolic,
                                         int *variant, int *n_variants, double *ms, double *lift_ms);
 /* The CUDA stream (cudaStream_t) the batch enqueues on, for event timing. */

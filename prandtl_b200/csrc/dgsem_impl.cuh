@@ -2106,10 +2106,22 @@ constexpr bool line_form() { return sizeof(Real) == 8 && (VC || !NS); }
 // lines per SM their longer serial chain counts.  SSP-RK3 step, general against
 // lines: vortex 32^2 N=3 22.5 / 25.8 us, N=4 24.9 / 39.1, 64^2 N=4 44.4 / 41.2,
 // 48^2 N=5 39.7 / 50.4, 64^2 N=5 63.7 / 53.1; at N=1 the lines are always ahead
-// (21.8 / 16.1).
-template <int DIM, int NP, typename Real>
+// (21.8 / 16.1).  In 3D they are at every size from 2^3 on.  Walls lengthen the
+// viscous chain most: from N=3 on its line lies at 21,000 lines there (LSRK4(5)
+// step 64^2 N=3 79.5 / 91.2, 72^2 112.2 / 111.7, 56^2 N=5 167 / 183, 64^2 191 / 184).
+template <int DIM, int NP, bool NS, typename Real>
 bool small_2d(const MeshDev &m) {
-    return DIM == 2 && NP > 2 && sizeof(Real) == 8 && (long long)m.E * NP < 15000;
+    return DIM == 2 && NP > 2 && sizeof(Real) == 8 && (long long)m.E * NP < (NS && m.bcs && NP > 3 ? 21000 : 15000);
+}
+// The same for the reference mode's Navier-Stokes, whose lines save more beside
+// the gradients.  LSRK4(5) step, gradients against lines, us: 32^2 N=3 57.9 / 72.3,
+// 56^2 69.3 / 76.4, 64^2 105.2 / 78.4; 32^2 N=4 65.2 / 86.6, 48^2 112.2 / 89.8;
+// 32^2 N=5 81.3 / 117.4, 48^2 159.0 / 124.6; ahead at every size at N <= 2
+// (N=2 8^2 59.5 / 56.8) and in 3D.  The RHS and the lifting both ask here: what
+// one writes the other reads.
+template <int DIM, int NP>
+bool ref_by_lines(const MeshDev &m, const PhysParams &P) {
+    return m.ref_lines && !P.blending && (DIM == 3 || NP <= 3 || (long long)m.E * NP >= (NP == 4 ? 13000 : 10000));
 }
 // non-affine meshes (m.ngeo set) run the per-node-geometry kernels (FP64, or FP32-bulk Euler)
 template <int DIM, int NP, bool NS, bool VC, typename Real>
@@ -2120,10 +2132,10 @@ cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams 
         else return cudaErrorNotSupported;
     }
     if constexpr (sizeof(Real) == 8 && NS && !VC) {   // reference mode: plain solves by lines
-        if (m.ref_lines && !P.blending) return rhs_line_launch<DIM, NP, true, false, false, true>(m, a, P, T, s);
+        if (ref_by_lines<DIM, NP>(m, P)) return rhs_line_launch<DIM, NP, true, false, false, true>(m, a, P, T, s);
     }
     if constexpr (line_form<NS, VC, Real>()) {   // by lines, but for the axisymmetric form
-        if (DIM == 3 || (!m.rad && !small_2d<DIM, NP, Real>(m))) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
+        if (DIM == 3 || (!m.rad && !small_2d<DIM, NP, NS, Real>(m))) return rhs_line_any<DIM, NP, NS>(m, a, P, T, s);
     }
     if constexpr (sizeof(Real) == 4 || (NS && !VC) || DIM == 2)
         return P.blending || m.bcs ? rhs_launch_np<DIM, NP, NS, VC, Real, true, false>(m, a, P, T, s)
@@ -2154,13 +2166,13 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
         else return cudaErrorNotSupported;
     }
     if constexpr (sizeof(Out) == 8 && !VC) {
-        if (m.ref_lines && !P.blending) return lift_line_launch<DIM, NP, false, Out, true>(m, a, P, T, s);
+        if (ref_by_lines<DIM, NP>(m, P)) return lift_line_launch<DIM, NP, false, Out, true>(m, a, P, T, s);
     }
     // the lines take the adjugate rows for the normals: in FP64 only where they are
     // the same within rounding (FP32's own rounding, 6e-8, covers the 1e-9 that
     // meshes may be off by)
     if constexpr (VC && sizeof(Out) == 8) {
-        if (!m.nor_rows || small_2d<DIM, NP, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
+        if (!m.nor_rows || small_2d<DIM, NP, true, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
     }
     if constexpr (VC)
         return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)

@@ -2123,6 +2123,20 @@ template <int DIM, int NP>
 bool ref_by_lines(const MeshDev &m, const PhysParams &P) {
     return m.ref_lines && !P.blending && (DIM == 3 || NP <= 3 || (long long)m.E * NP >= (NP == 4 ? 13000 : 10000));
 }
+// And for the FP32-bulk lifting on one mesh, whose lanes form their nodes'
+// entropy variables in FP64 one after the other.  LSRK4(5) step, node by node
+// against lines, us: 3D 8^3 N=3 85.0 / 91.7, 10^3 95.1 / 94.7, 12^3 109 / 106;
+// 8^3 N=4 111 / 116, 10^3 146 / 134; 4^3 N=5 89 / 120, 8^3 122 / 135, 10^3 214 / 210;
+// 2D 24^2 N=3 44.1 / 53.5, 64^2 55.9 / 61.6, 96^2 98.4 / 93.9; 32^2 N=4 55.8 / 62.1,
+// 64^2 100.0 / 103.6, 96^2 196 / 179; 32^2 N=5 66.5 / 75.3, 48^2 91.4 / 84.1; level
+// or behind at N <= 2 (3D 10^3 N=2 79.0 / 73.4).  A batch keeps to lines (many
+// small solves fill the device, and what a solve runs must not depend on the
+// others): one 4^3 N=5 solve alone in a batch 168 us a step against 123, 32 of
+// them level, the 96 of an ensemble 1.12 times as fast.
+template <int DIM, int NP>
+bool few_lines_fp32(const MeshDev &m) {
+    return NP > 3 && (long long)m.E * (ipow(NP, DIM) / NP) < (DIM == 2 && NP == 6 ? 10000 : 20000);
+}
 // non-affine meshes (m.ngeo set) run the per-node-geometry kernels (FP64, or FP32-bulk Euler)
 template <int DIM, int NP, bool NS, bool VC, typename Real>
 cudaError_t rhs_launch_any(const MeshDev &m, const RhsArgs &a, const PhysParams &P, const OpTables &T,
@@ -2171,8 +2185,9 @@ cudaError_t lift_launch_any(const MeshDev &m, const LiftArgs &a, const PhysParam
     // the lines take the adjugate rows for the normals: in FP64 only where they are
     // the same within rounding (FP32's own rounding, 6e-8, covers the 1e-9 that
     // meshes may be off by)
-    if constexpr (VC && sizeof(Out) == 8) {
-        if (!m.nor_rows || small_2d<DIM, NP, true, Out>(m)) return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
+    if constexpr (VC) {
+        if (sizeof(Out) == 8 ? !m.nor_rows || small_2d<DIM, NP, true, Out>(m) : few_lines_fp32<DIM, NP>(m))
+            return lift_launch_np<DIM, NP, Out, VC, false>(m, a, P, T, s);
     }
     if constexpr (VC)
         return m.bcs ? lift_line_launch<DIM, NP, true, Out>(m, a, P, T, s)

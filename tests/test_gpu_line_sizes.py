@@ -45,3 +45,28 @@ def test_walls(oracle_mod, order, n, blending):
     op = DGSEMOperator(mesh, quirks="fixed", parabolic=True, blending=blending, **kw)
     assert normalized_error(op.Mult(u, np.empty_like(u)), r["dudt"], 4) <= 1e-12
     op.close()
+
+
+# FP32-bulk lifting: just below and above 20,000 lines (2D N=5: 10,000), and N <= 2 by lines
+FP32 = [(2, 2, (9, 7)), (2, 3, (70, 71)), (2, 3, (71, 73)), (2, 4, (60, 65)), (2, 4, (60, 67)), (2, 5, (40, 41)),
+        (2, 5, (40, 43)), (3, 1, (3, 3, 2)), (3, 2, (3, 3, 2)), (3, 3, (10, 11, 11)), (3, 3, (10, 11, 12)),
+        (3, 4, (9, 9, 9)), (3, 4, (9, 9, 10)), (3, 5, (8, 8, 8)), (3, 5, (8, 8, 9))]
+
+
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("dim,order,n", FP32)
+def test_fp32_lifting(dim, order, n, walls):
+    """Within the FP32-bulk form's bound of the FP64 right-hand side, 2e-3 in relative L2."""
+    from prandtl_b200.operator import DGSEMOperator
+    from test_gpu_fp32 import rel_l2
+    kw = dict(mu=0.01, R_gas=1.0, parabolic=True, quirks="fixed")
+    if walls:
+        kw["bcs"] = [("noslip_adiabatic", dict(wall_vel=(0.1,) + (0.0,) * (dim - 1), heat_flux=0.02)), ("outflow",)]
+    mesh = periodic_box(dim, n, order, 0.0, tuple(0.5 * c for c in n), bcs=[None] * (2 * dim - 2) + [0, 1] if walls else None)
+    u = cases.perturbed(mesh, cases.free_stream(mesh, p=1.5), amp=0.1, seed=order)
+    out = []
+    for precision in ("fp64", "fp32"):
+        op = DGSEMOperator(mesh, precision=precision, **kw)
+        out.append(op.Mult(u, np.empty_like(u)))
+        op.close()
+    assert max(rel_l2(out[1], out[0], mesh.num_fields)) <= 2e-3

@@ -56,7 +56,9 @@ struct LineShape {
     // 3D Np = 5, 126 at Np = 3, 252 of 256 at Np = 6
     static constexpr int THREADS = (!WARP && NL > 32) ? 256 : 128;
     static constexpr int EPB = WARP ? (THREADS / 32) * EPW : THREADS / NL;
+    static_assert(EPB >= 1 && EPB * NL <= THREADS && THREADS % 32 == 0 && EPW * NL <= 32, "lanes of a CTA and of a warp");
 };
+constexpr size_t MAX_SMEM = 227 * 1024;   // shared memory a CTA can have
 // The right-hand side's shared area of an element.
 template <int DIM, int NP>
 struct RhsLineShape : LineShape<DIM, NP> {
@@ -69,6 +71,8 @@ struct RhsLineShape : LineShape<DIM, NP> {
     // adj(J) and det J
     static constexpr int NBR = (K + L::NF) * L::ROW, NOR = NBR + 4 * DIM, GEO = NOR + 2 * DIM * (DIM + 1);
     static constexpr int PER_ELEM = L::padded(GEO + DIM * DIM + 1);
+    static_assert(GEO + DIM * DIM + 1 <= PER_ELEM && 3 * L::NL <= L::NF * L::ROW, "an element's shared area");
+    static_assert(sizeof(double) * L::EPB * PER_ELEM + CTX_RESERVE <= MAX_SMEM, "a CTA's shared memory");
 };
 
 // Resident CTAs the register budget is sized for: 168 registers a thread.  A
@@ -806,6 +810,8 @@ struct LiftLineShape : LineShape<DIM, NP, W> {
     // then the neighbour table (two ints a face), adj(J) and 1 / det J
     static constexpr int NBR = DIM * L::NF * L::ROW, GEO = NBR + 4 * DIM * 4 / (int)sizeof(W);
     static constexpr int PER_ELEM = L::padded(GEO + DIM * DIM + 1);
+    static_assert((GEO - NBR) * sizeof(W) >= 4 * DIM * sizeof(int) && GEO + DIM * DIM + 1 <= PER_ELEM, "an element's shared area");
+    static_assert(sizeof(W) * L::EPB * PER_ELEM + CTX_RESERVE <= MAX_SMEM, "a CTA's shared memory");
 };
 // D(i, l) in the working precision.
 template <typename W>

@@ -857,19 +857,22 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
 #pragma unroll
         for (int f = 0; f < NF; ++f) { dUi[k][f] = 0; dUv[k][f] = 0; }
 
-    // VC: row f (1..NF-1) of direction r at node n of element el.  Affine elements:
-    // in line order (lift_line_element), per element [DIM][NF-1][position along
-    // the line][line]; non-affine: [DIM][NF-1][Ndof]
-    auto visc_at = [&](long long el, int r, int f, int n) -> long long {
-        if (CURV) return (r * (NF - 1) + f - 1) * Ndof + el * ND + n;
-        int c[3];
-        node_coords<NP>(n, c);
-        return ((el * DIM + r) * (NF - 1) + f - 1) * ND + c[r] * S::NLINE + line_index<DIM, NP>(r, c);
-    };
+    // VC: rows f = 1..NF-1 of the DIM directions, in line order (lift_line_element),
+    // per element [DIM][NF-1][position along the line][line]; non-affine:
+    // [DIM][NF-1][Ndof].  Element el's row (r, f) starts at el * row_e + (r (NF-1) + f-1) * row_f.
+    constexpr int row_e = CURV ? ND : DIM * (NF - 1) * ND;
+    const long long row_f = CURV ? Ndof : (long long)ND;
     // ---- NS: contravariant viscous flux of every own node (flux_mat = adj * Fv^T, :632)
-    if constexpr (NS && VC && !LY::LINE) {   // (line tasks read their rows themselves)
+    // The rows pass through shared memory, their loads in flight before the two-point
+    // fluxes; line tasks that read theirs from global memory after them waited for it
+    // (FP32 batch RHS, 3D N=2 124 -> 117 us, N=3 84 -> 80, N=4 82 -> 77, N=5 109 -> 98).
+    // The three lines of a 2D Np = 3 element are too few for that to pay (128^2 FP32
+    // step 108 us as it is, 119 through shared memory).
+    constexpr bool STAGED = !(LY::LINE && DIM == 2 && NP == 3);
+    if constexpr (NS && VC && STAGED) {
         // formed by the lifting: rows f = 1..NF-1 of adj * Fv^T (the mass row is zero);
-        // each lane's loads are all issued before the stores
+        // each lane's loads are all issued before the stores; a lane takes the positions
+        // li, li + GS, ... of the rows
         Real vrow[NPL][DIM][NF - 1];
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
@@ -878,16 +881,20 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
             for (int r = 0; r < DIM; ++r)
 #pragma unroll
                 for (int f = 1; f < NF; ++f)
-                    vrow[k][r][f - 1] = n < ND ? __ldg(grad + visc_at(e, r, f, n)) : Real(0);
+                    vrow[k][r][f - 1] = n < ND ? __ldg(grad + (long long)e * row_e + (r * (NF - 1) + f - 1) * row_f + n) : Real(0);
         }
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
             const int n = li + k * GS;
             if (n < ND) {
 #pragma unroll
-                for (int r = 0; r < DIM; ++r)
+                for (int r = 0; r < DIM; ++r) {
+                    int base, stride;
+                    line_base<DIM, NP>(r, n % S::NLINE, base, stride);
+                    const int at = CURV ? n : base + n / S::NLINE * stride;
 #pragma unroll
-                    for (int f = 1; f < NF; ++f) sV[(r * LY::VROWS + f - LY::VOFF) * ND + n] = vrow[k][r][f - 1];
+                    for (int f = 1; f < NF; ++f) sV[(r * LY::VROWS + f - LY::VOFF) * ND + at] = vrow[k][r][f - 1];
+                }
             }
         }
     } else if constexpr (NS && !VC) {
@@ -1004,8 +1011,9 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
             for (int l = 0; l < NP; ++l)
 #pragma unroll
                 for (int f = 1; f < NF; ++f)
-                    vv[l][f - 1] = VC ? __ldg(grad + (((long long)e * DIM + dir) * (NF - 1) + f - 1) * ND + l * S::NLINE + ln)
-                                      : sV[(dir * NF + f) * ND + base + l * stride];
+                    vv[l][f - 1] = !VC || STAGED ? sV[(dir * NF + f) * ND + base + l * stride]
+                                                 : __ldg(grad + (long long)e * row_e + (dir * (NF - 1) + f - 1) * row_f +
+                                                         l * S::NLINE + ln);
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
                 Real *out = sV + dir * NF * ND + base + i * stride;
@@ -1230,8 +1238,8 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
         const int lf = it / NFN, fa = it - lf * NFN;
         const int no = face_node<DIM, NP>(lf, fa);
         x.t = NBR_SMEM ? sNbr[lf] : __ldg(a.nbr + (long long)e * (2 * DIM) + lf);
-        const long long en = x.t.x < 0 ? e : x.t.x;
-        const int nn = x.t.x < 0 ? no : face_node<DIM, NP>(x.t.y, fa);
+        const long long en = x.t.x < 0 ? e : x.t.x;   // (boundary faces: the own trace and rows)
+        const int lfn = x.t.x < 0 ? lf : x.t.y, nn = x.t.x < 0 ? no : face_node<DIM, NP>(x.t.y, fa);
         const long long gs = en * ND + nn;
 #pragma unroll
         for (int f = 0; f < NF; ++f) x.s[f] = __ldg(a.u + f * Ndof + gs);
@@ -1240,11 +1248,16 @@ __device__ __forceinline__ void rhs_element(const ElemIO &a, const PhysParams &P
             x.nb[q] = CURV ? __ldg(a.fnn + ((long long)x.t.z * NFN + fa) * DIM + q)
                            : __ldg(a.fnor + (long long)x.t.z * DIM + q);
         if constexpr (NS && VC) {
-            const int dd = lf >> 1, dn = x.t.x < 0 ? dd : x.t.y >> 1;
+            // in line order a face's nodes are the lines of its direction, at their first or
+            // last position
+            auto row = [&](long long el, int l, long long g) -> long long {
+                return (l >> 1) * (NF - 1) * row_f + (CURV ? g : el * row_e + (l & 1) * (NP - 1) * S::NLINE + fa);
+            };
+            const long long ro = row(e, lf, (long long)e * ND + no), rn = row(en, lfn, gs);
 #pragma unroll
-            for (int f = 1; f < NF; ++f) {
-                x.vo[f - 1] = __ldg(grad + visc_at(e, dd, f, no));
-                x.vn[f - 1] = __ldg(grad + visc_at(en, dn, f, nn));
+            for (int f = 0; f < NF - 1; ++f) {
+                x.vo[f] = __ldg(grad + ro + f * row_f);
+                x.vn[f] = __ldg(grad + rn + f * row_f);
             }
         }
     };

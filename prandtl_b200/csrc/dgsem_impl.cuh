@@ -2145,10 +2145,15 @@ bool ref_by_lines(const MeshDev &m, const PhysParams &P) {
 // or behind at N <= 2 (3D 10^3 N=2 79.0 / 73.4).  A batch keeps to lines (many
 // small solves fill the device, and what a solve runs must not depend on the
 // others): one 4^3 N=5 solve alone in a batch 168 us a step against 123, 32 of
-// them level, the 96 of an ensemble 1.12 times as fast.
+// them level, the 96 of an ensemble 1.12 times as fast.  Boundary faces lengthen
+// the lines' chain most: there they are ahead from 70,000 lines on, at N=2 and in
+// 2D at N=5 from 20,000 (128^2 N=3 176 / 194, N=4 64^2 110 / 125, 128^2 339 / 336;
+// 3D 12^3 N=5 379 / 395, 18^3 N=3 354 / 339; 24^3 N=2 508 / 484; 2D 64^2 N=5 161 / 156).
 template <int DIM, int NP>
 bool few_lines_fp32(const MeshDev &m) {
-    return NP > 3 && (long long)m.E * (ipow(NP, DIM) / NP) < (DIM == 2 && NP == 6 ? 10000 : 20000);
+    const long long lines = (long long)m.E * (ipow(NP, DIM) / NP);
+    if (m.bcs) return lines < (NP == 3 || (DIM == 2 && NP == 6) ? 20000 : 70000);
+    return NP > 3 && lines < (DIM == 2 && NP == 6 ? 10000 : 21000);
 }
 // non-affine meshes (m.ngeo set) run the per-node-geometry kernels (FP64, or FP32-bulk Euler)
 template <int DIM, int NP, bool NS, bool VC, typename Real>

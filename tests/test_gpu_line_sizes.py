@@ -47,10 +47,13 @@ def test_walls(oracle_mod, order, n, blending):
     op.close()
 
 
-# FP32-bulk lifting: just below and above 20,000 lines (2D N=5: 10,000), and N <= 2 by lines
-FP32 = [(2, 2, (9, 7)), (2, 3, (70, 71)), (2, 3, (71, 73)), (2, 4, (60, 65)), (2, 4, (60, 67)), (2, 5, (40, 41)),
-        (2, 5, (40, 43)), (3, 1, (3, 3, 2)), (3, 2, (3, 3, 2)), (3, 3, (10, 11, 11)), (3, 3, (10, 11, 12)),
-        (3, 4, (9, 9, 9)), (3, 4, (9, 9, 10)), (3, 5, (8, 8, 8)), (3, 5, (8, 8, 9))]
+# FP32-bulk lifting: just below and above 21,000 lines (2D N=5: 10,000), and N <= 2 by lines;
+# with walls 70,000 (N=2 and 2D N=5: 20,000)
+FP32 = [(2, 1, (185, 189)), (2, 1, (187, 189)), (2, 2, (80, 83)), (2, 2, (80, 84)), (2, 3, (130, 134)), (2, 3, (130, 135)),
+        (2, 5, (55, 60)), (2, 5, (55, 61)), (3, 2, (13, 13, 13)), (3, 2, (13, 13, 14)), (3, 3, (16, 16, 17)), (3, 3, (16, 17, 17)),
+        (2, 2, (9, 7)), (2, 3, (70, 74)), (2, 3, (71, 75)), (2, 4, (60, 69)), (2, 4, (60, 71)), (2, 5, (40, 41)),
+        (2, 5, (40, 43)), (3, 1, (3, 3, 2)), (3, 2, (3, 3, 2)), (3, 3, (10, 11, 11)), (3, 3, (11, 11, 11)),
+        (3, 4, (9, 9, 10)), (3, 4, (9, 10, 10)), (3, 5, (8, 8, 9)), (3, 5, (8, 9, 9))]
 
 
 @pytest.mark.parametrize("walls", [False, True])

@@ -870,13 +870,13 @@ def main():
         lby = E_dom * nd_dom * (5 * 8 + 3 * 4 * 4)
         ltr = measured_traffic().get(f"lift_batch_N{dom_order}_fp32")
         roofline["lift"] = {
-            "kernel": f"lift_batch_kernel<3, N={dom_order}, float> (all N={dom_order} members, one stage)",
+            "kernel": f"lift_line_batch_kernel<3, N={dom_order}, float> (all N={dom_order} members, one stage)",
             "bound": "hbm", "algorithmic_bytes_per_launch": lby, "avg_launch_ms": t_lift * 1e3,
             "achieved_gbs": lby / t_lift / 1e9, "peak_gbs": hbm_peak, "frac": lby / t_lift / 1e9 / hbm_peak,
             "peak_source": hbm_src,
             "traffic": ltr["bytes_per_element"] * E_dom if ltr else None,
             "traffic_source": ("ncu dram bytes of this kernel on the N=5 members of a 24-member ensemble, scaled by "
-                               "elements (ncu summary lift_batch_kernel_N5_fp32_ncu under profiles/)") if ltr else None}
+                               "elements (ncu summary line_kernels_ncu under profiles/)") if ltr else None}
         ivortex32 = run_ivortex32(torch) if not args.no_configs else None
         kh256 = run_kh256(torch) if not args.no_configs else None
         ramp = run_ramp(torch) if not args.no_configs else None

@@ -4,8 +4,10 @@
 //
 // The FP64 RHS on affine meshes and the liftings with contravariant viscous
 // rows run by lines (dgsem_line.cuh).  The general form below runs the others:
-// the FP32-bulk RHS, non-affine and axisymmetric meshes, and Navier-Stokes with
-// gradients (the reference mode in batches, in FP32, with blending or boundaries).
+// the FP32-bulk RHS, non-affine and axisymmetric meshes, Navier-Stokes with
+// gradients (the reference mode in batches, in FP32, with blending or boundaries),
+// and operators on meshes with few lines (small_2d, ref_by_lines, few_lines_fp32);
+// its lifting also FP64 meshes whose normals are not their adjugate rows.
 //
 // RHS: one lane group (a warp, or a power-of-two part of one for small
 // elements) per element.  Everything an element needs stays in shared memory
@@ -2111,7 +2113,11 @@ cudaError_t rhs_launch_np(const MeshDev &m, const RhsArgs &a, const PhysParams &
     return cudaErrorInvalidValue;
 }
 // The FP64 forms on affine meshes run by lines (dgsem_line.cuh), but for
-// Navier-Stokes with gradients, the axisymmetric form and small 2D meshes.
+// Navier-Stokes with gradients, the axisymmetric form and small 2D meshes.  In
+// batches at every size: few small 2D solves are slower there (one 16^2 solve,
+// general against lines, LSRK4(5) step: N=4 Euler 52 / 58 us, viscous 78 / 104; N=5
+// viscous 91 / 130), many are faster (32 of them: N=4 166 / 91 and 289 / 162), and
+// what a solve runs must not depend on the others.
 template <bool NS, bool VC, typename Real>
 constexpr bool line_form() { return sizeof(Real) == 8 && (VC || !NS); }
 // Small 2D meshes stay with the general form in FP64: it gives an element's

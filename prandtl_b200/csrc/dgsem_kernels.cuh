@@ -171,8 +171,9 @@ cudaError_t batch_launch_step_end(BatchInst *tab, const int *live, const int *n_
 
 // Per-(dim, working precision, physics) dispatchers, one translation unit each.
 // VC (Navier-Stokes only): the lifting emits the contravariant viscous fluxes
-// adj * Fv^T, rows 1..NF-1, as [DIM][NF-1][Ndof] in the gradient buffer, and
-// the RHS reads them instead of evaluating viscous fluxes from gradients.
+// adj * Fv^T, rows 1..NF-1, into the gradient buffer (affine elements: in line
+// order, [E][DIM][NF-1][position][line]; else [DIM][NF-1][Ndof]), and the RHS
+// reads them instead of evaluating viscous fluxes from gradients.
 template <int DIM, typename Real, bool NS, bool VC>
 cudaError_t rhs_dispatch(int order, const MeshDev &m, const RhsArgs &a, const PhysParams &P,
                          const OpTables &T, cudaStream_t s);

@@ -15,7 +15,7 @@
 // pair, no two-point or face flux goes through shared memory, every lane has
 // work in every phase and boundary and blending code is compiled in only where
 // it is used: half the warp instructions (157 M -> 73 M at 32^3 Np = 4).  What
-// bounds it now is FP64 issue (49 % of the pipe) and the latency of the global
+// bounds it now is FP64 issue (53 % of the pipe) and the latency of the global
 // loads at 12 warps per SM.  Measured, one launch:
 //   3D Np = 4 Navier-Stokes, 32^3 elements   324 -> 147 us
 //   3D Np = 5 Navier-Stokes, 15^3            103 ->  49 us
